@@ -13,14 +13,16 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libgsvit_b200.so")
 BUILD = os.path.join(HERE, "_build")
 
-SOURCES = ["fdtd_kernels.cu", "fdtd_bulk.cu", "fdtd_adjoint.cu", "fdtd_api.cu", "plan_host.cpp"]
-HEADERS = ["fdtd_internal.h", "fdtd_device.cuh", "fdtd_cells.cuh", "fdtd_cpgroup.cuh", "fdtd_kernels.cuh", "fdtd_bulk.cuh",
+SOURCES = ["fdtd_kernels.cu", "fdtd_bulk.cu", "fdtd_flat.cu", "fdtd_flat_f32.cu", "fdtd_flat_f16.cu",
+           "fdtd_flat_bf16.cu", "fdtd_flat_f64.cu", "fdtd_adjoint.cu", "fdtd_api.cu", "plan_host.cpp"]
+HEADERS = ["fdtd_internal.h", "fdtd_device.cuh", "fdtd_cpgroup.cuh", "fdtd_kernels.cuh", "fdtd_bulk.cuh", "fdtd_flat.cuh", "fdtd_flat_kernels.cuh",
            "fdtd_adjoint.cuh", "plan_host.h", os.path.join("..", "..", "include", "gsvit_b200.h")]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -42,7 +44,7 @@ def _stale(target: str, deps) -> bool:
 def build(force: bool = False, ptxas_verbose: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
     hdrs = [os.path.normpath(os.path.join(CSRC, h)) for h in HEADERS]
-    objs = []
+    objs, jobs = [], []
     common = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fopenmp", "--expt-relaxed-constexpr"]
     for src in SOURCES:
         sp = os.path.join(CSRC, src)
@@ -52,7 +54,9 @@ def build(force: bool = False, ptxas_verbose: bool = False) -> str:
             cmd = [nvcc()] + ARCH + common + ["-c", sp, "-o", obj]
             if src.endswith(".cu") and ptxas_verbose:
                 cmd += ["-Xptxas", "-v"]
-            subprocess.check_call(cmd)
+            jobs.append(cmd)
+    with ThreadPoolExecutor(max_workers=max(1, min(len(jobs), os.cpu_count() or 1))) as ex:
+        list(ex.map(subprocess.check_call, jobs))   # raises the first failure
     if force or _stale(OUT, objs):
         tmp = OUT + ".tmp"
         subprocess.check_call([nvcc()] + ARCH + ["-shared", "-o", tmp] + objs + ["-lgomp", "-lcudart"])

@@ -23,8 +23,6 @@
 
 namespace {
 
-enum { X0 = 0, XN = 1, Y0 = 2, YN = 3, Z0 = 4, ZN = 5 };
-
 __device__ __forceinline__ void cell_ijk(const DevPlan &P, int64_t c, int &i, int &j, int &k)
 {
     k = (int)(c % P.zr);

@@ -22,6 +22,7 @@
 #include "../../include/gsvit_b200.h"
 #include "fdtd_internal.h"
 #include "fdtd_bulk.cuh"
+#include "fdtd_flat.cuh"
 #include "fdtd_kernels.cuh"
 #include "fdtd_adjoint.cuh"
 #include "plan_host.h"
@@ -95,13 +96,11 @@ struct fdtd_plan {
     const float **d_fieldptrs[2] = {nullptr, nullptr};   // device copies of fields[s]
     int *d_step = nullptr;
     int host_step = 0;
-    // work decomposition: slab kernels (CPML slabs, grid edges) and TMA bulk kernel
-    SlabBox *d_boxes = nullptr;     // slab boxes (numbered one cell per thread)
-    int nboxes = 0;
-    long long nslab_blocks = 0;
-    SlabBox *d_boxes4 = nullptr;    // the same numbered in 4-cell groups (H kernel), when all are 4-aligned
-    long long nslab_blocks4 = 0;
-    SlabLists slabs{};              // the lists above plus the E split (runs with / without dispersive cells)
+    // work decomposition: the TMA bulk kernel on an interior box (large grids)
+    // and the flat kernels on the rest, or the flat kernels on the whole grid
+    int fwidth = 1;                          // cells per thread of the flat kernels
+    std::vector<FlatBlock> h_flat;           // host copy of their block list (batched launches)
+    FlatList flat, flat_in, flat_sp;         // all blocks; the plain interior's and the rest (fdtd_step_profile)
     BulkItem *d_bulk = nullptr;
     int nbulk = 0;
     bool bulk_on = false;
@@ -123,9 +122,6 @@ struct fdtd_plan {
     const int *batch_err = nullptr;       // the batch's error word, for an instance of a batch
     bool failed = false;                  // an expired wait was reported: the plan only accepts destroy
     int region[6] = {0, 0, 0, 0, 0, 0};   // bulk box Xlo Xhi Ylo Yhi Zlo Zhi
-    std::vector<SlabBox> h_boxes;         // host copies of the work lists (batched launches)
-    std::vector<SlabBox> h_eboxes;        // E runs with a dispersive cell (every box when unsplit)
-    std::vector<SlabBox> h_epboxes;       // E runs without one
     std::vector<BulkItem> h_bulk;
     int bulk_len = 0;                     // planes per bulk item
     int tsf_cells = 0;                    // face cells of the TSF correction tables
@@ -199,7 +195,7 @@ int launch_tile_kind(fdtd_plan *P, const DevPlan &d, int in, int kind, cudaStrea
 
 // the Yee/CPML/TSF/ADE part of one step: the TMA tiles (bulk, then the CPML
 // tiles; they touch disjoint cells and read only the input set), or, for
-// plans without them, the bulk box and the slab kernels
+// plans without them, the bulk box and the flat kernels, or the flat kernels alone
 int launch_fused(fdtd_plan *P, int in, cudaStream_t st)
 {
     DevPlan d = plan_for(P, in);
@@ -228,33 +224,28 @@ int launch_fused(fdtd_plan *P, int in, cudaStream_t st)
         }
         return FDTD_OK;
     }
-    if (P->bulk_on && P->side[TILE_CPX] && P->slabs.hblocks > 0) {
-        // the slab H kernel beside the bulk kernel (disjoint cells, input set
-        // only); the slab E kernels after both: they read H^{n+1/2} the bulk
-        // kernel wrote next to the slabs
+    if (P->bulk_on) {
+        // the flat H kernel beside the bulk kernel (disjoint cells, input set
+        // only); the flat E kernel after both: it reads H^{n+1/2} the bulk
+        // kernel wrote next to its boxes
         if ((e = cudaEventRecord(P->ev_fork, st)) != cudaSuccess ||
             (e = cudaStreamWaitEvent(P->side[TILE_CPX], P->ev_fork, 0)) != cudaSuccess)
-            return fail(FDTD_E_CUDA, std::string("slab fork: ") + cudaGetErrorString(e));
-        e = launch_slab_steps(d, P->slabs, P->hp.has_ade, P->hp.maxpoles, P->storage, P->side[TILE_CPX], 1);
-        if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("slab step launch: ") + cudaGetErrorString(e));
+            return fail(FDTD_E_CUDA, std::string("flat fork: ") + cudaGetErrorString(e));
+        e = launch_flat_h(d, P->flat, P->fwidth, P->storage, P->side[TILE_CPX]);
+        if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("flat H launch: ") + cudaGetErrorString(e));
         if ((e = cudaEventRecord(P->ev_join[TILE_CPX], P->side[TILE_CPX])) != cudaSuccess)
-            return fail(FDTD_E_CUDA, std::string("slab join: ") + cudaGetErrorString(e));
+            return fail(FDTD_E_CUDA, std::string("flat join: ") + cudaGetErrorString(e));
         e = launch_tiles(TILE_BULK, d, P->bmaps[in], P->d_bulk, P->nbulk, P->d_err, P->hp.has_ade, P->hp.maxpoles,
                          P->storage, 0, st);
         if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("bulk step launch: ") + cudaGetErrorString(e));
         if ((e = cudaStreamWaitEvent(st, P->ev_join[TILE_CPX], 0)) != cudaSuccess)
-            return fail(FDTD_E_CUDA, std::string("slab join: ") + cudaGetErrorString(e));
-        e = launch_slab_steps(d, P->slabs, P->hp.has_ade, P->hp.maxpoles, P->storage, st, 2);
-        if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("slab step launch: ") + cudaGetErrorString(e));
-        return FDTD_OK;
+            return fail(FDTD_E_CUDA, std::string("flat join: ") + cudaGetErrorString(e));
+    } else {
+        e = launch_flat_h(d, P->flat, P->fwidth, P->storage, st);
+        if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("flat H launch: ") + cudaGetErrorString(e));
     }
-    if (P->bulk_on) {   // first: the slab E update reads H^{n+1/2} the bulk kernel wrote next to the slabs
-        e = launch_tiles(TILE_BULK, d, P->bmaps[in], P->d_bulk, P->nbulk, P->d_err, P->hp.has_ade, P->hp.maxpoles,
-                         P->storage, 0, st);
-        if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("bulk step launch: ") + cudaGetErrorString(e));
-    }
-    e = launch_slab_steps(d, P->slabs, P->hp.has_ade, P->hp.maxpoles, P->storage, st);
-    if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("slab step launch: ") + cudaGetErrorString(e));
+    e = launch_flat_e(d, P->flat, P->fwidth, P->hp.has_ade, P->hp.maxpoles, P->storage, st);
+    if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("flat E launch: ") + cudaGetErrorString(e));
     return FDTD_OK;
 }
 
@@ -445,7 +436,7 @@ int build_tiles(fdtd_plan *P, const HostPlan &hp, DevPlan &d, const uint8_t *cls
     const bool bulk = bi0 < bi1 && bj0 < bj1 && bk0 < bk1;
     // design cells (per-cell E coefficients) are handled by the bulk layout
     // only: a plan whose design cells reach outside the interior box keeps the
-    // slab kernels
+    // flat kernels
     if (hp.design && !(bulk && hp.abox[0] >= bi0 && hp.abox[1] <= bi1 && hp.abox[2] >= bj0 && hp.abox[3] <= bj1 &&
                        hp.abox[4] >= bk0 && hp.abox[5] <= bk1)) {
         P->tiles_on = false;
@@ -526,6 +517,132 @@ int build_tiles(fdtd_plan *P, const HostPlan &hp, DevPlan &d, const uint8_t *cls
     e = bulk_configure();
     if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("tile kernel shared memory: ") + cudaGetErrorString(e));
     return FDTD_OK;
+}
+
+std::vector<FlatBlock> flat_emit(const std::vector<FlatBlock> &pieces)
+{
+    std::vector<FlatBlock> out;
+    for (FlatBlock B : pieces)
+        for (B.t0 = 0; B.t0 < B.total; B.t0 += FLAT_NT) out.push_back(B);
+    return out;
+}
+
+// The flat kernels' blocks: the grid without [lo, hi) as boxes of every
+// combination of low slab, middle and high slab on the three axes, and, with
+// `inner`, that box as well, which then holds plain cells only.  Each box is split along k into runs of k groups of one class
+// and runs of several (runs of one class shorter than 8 planes join them):
+// blocks of one class need no class map, and know their dispersive state
+// before they read a field.  Boxes are cut along i into pieces of a few
+// blocks, and the pieces ordered by i.
+std::vector<FlatBlock> flat_blocks(const HostPlan &hp, const DevPlan &d, const int lo[3], const int hi[3], bool inner, int V)
+{
+    const int res[3] = {hp.xr, hp.yr, hp.zr};
+    std::vector<FlatBlock> pieces;   // one entry a piece
+    // cls: the class of every cell, or -1
+    auto push = [&](const int a[3], const int b[3], bool ade, int cls) {
+        int flags = ade ? FB_ADE : 0, axes = 0;
+        bool rim = false;   // a grid edge without CPML
+        for (int ax = 0; ax < 3; ax++) {
+            const int dl = d.cp_d[2 * ax], dh = d.cp_d[2 * ax + 1];
+            if (a[ax] < dl || b[ax] > res[ax] - dh) { flags |= (FB_X << ax) | FB_EDGE; axes++; }
+            if (a[ax] == 0 || b[ax] == res[ax]) flags |= FB_EDGE;
+            rim = rim || (a[ax] == 0 && !dl) || (b[ax] == res[ax] && !dh);
+            // a slab of each side in one box (a short axis)
+            rim = rim || (a[ax] < dl && b[ax] > res[ax] - dh);
+        }
+        if (cls >= 0) {
+            const unsigned f = hp.classes[cls].flags, own = f & (CF_ADE_BRANCH | CF_ADE_X | CF_ADE_Y | CF_ADE_Z);
+            if (!(f & (CF_PEC_X | CF_PEC_Y | CF_PEC_Z | CF_DESIGN)) &&
+                (!own || own == (CF_ADE_BRANCH | CF_ADE_X | CF_ADE_Y | CF_ADE_Z))) {
+                flags |= FB_ONE;
+                if (axes == 1 && !rim) flags |= FB_SPEC;
+            }
+        }
+        // TSF corrections touch cells in [t0 - 1, t1] on every axis (tsf_add_h/e)
+        bool meets = d.tsf_on != 0;
+        for (int ax = 0; ax < 3; ax++) meets = meets && a[ax] <= d.t1[ax] && b[ax] >= d.t0[ax];
+        if (meets) flags |= FB_TSF;
+        FlatBlock B;
+        std::memset(&B, 0, sizeof(B));
+        B.j0 = a[1]; B.k0 = a[2];
+        B.nk = (b[2] - a[2]) / V;
+        B.nj = b[1] - a[1];
+        B.flags = flags;
+        B.cls = (int16_t)std::max(cls, 0);
+        unsigned mk, mj;
+        int sk, sj;
+        flat_magic((unsigned)B.nk, &mk, &sk);
+        flat_magic((unsigned)B.nj, &mj, &sj);
+        B.mk = mk; B.mj = mj;
+        B.sk = (int8_t)sk; B.sj = (int8_t)sj;
+        const long long plane = (long long)B.nk * B.nj;   // groups a plane (< 2^31)
+        const int step = (int)std::max(1LL, std::min<long long>(b[0] - a[0], 8 * FLAT_NT / plane));
+        for (int i = a[0]; i < b[0]; i += step) {
+            B.i0 = i;
+            B.total = (unsigned)(plane * (std::min(b[0], i + step) - i));
+            pieces.push_back(B);
+        }
+    };
+    auto box = [&](const int a[3], const int b[3]) {
+        if (a[0] >= b[0] || a[1] >= b[1] || a[2] >= b[2]) return;
+        const int nz = b[2] - a[2], ng = nz / V;
+        std::vector<int> cls(ng, -2), disp(ng, 0);   // class of the k group's cells: -2 none seen, -1 several
+#pragma omp parallel for schedule(static)
+        for (int i = a[0]; i < b[0]; i++) {
+            std::vector<int> mc(nz, -2), md(nz, 0);
+            for (int j = a[1]; j < b[1]; j++) {
+                const uint8_t *row = &hp.cls[((size_t)i * res[1] + j) * res[2] + a[2]];
+                for (int k = 0; k < nz; k++) {
+                    const int c = row[k];
+                    mc[k] = mc[k] == -2 || mc[k] == c ? c : -1;
+                    md[k] |= (hp.classes[c].flags & CF_ADE_BRANCH) != 0;
+                }
+            }
+#pragma omp critical(flat_runs)
+            for (int k = 0; k < nz; k++) {
+                int &c = cls[k / V];
+                c = c == -2 || c == mc[k] ? mc[k] : -1;
+                disp[k / V] |= md[k];
+            }
+        }
+        const int least = 8 / V;
+        for (int g = 0; g < ng;) {   // short runs of one class join the mixed ones
+            int e = g;
+            while (e < ng && cls[e] == cls[g]) e++;
+            if (e - g < least && e - g < ng)
+                for (int r = g; r < e; r++) cls[r] = -1;
+            g = e;
+        }
+        for (int g = 0; g < ng;) {
+            int e = g, ade = 0;
+            while (e < ng && cls[e] == cls[g]) ade |= disp[e++];
+            const int x[3] = {a[0], a[1], a[2] + g * V}, y[3] = {b[0], b[1], a[2] + e * V};
+            push(x, y, ade != 0, cls[g]);
+            g = e;
+        }
+    };
+    if (lo[0] >= hi[0] || lo[1] >= hi[1] || lo[2] >= hi[2]) {
+        const int z[3] = {0, 0, 0};
+        box(z, res);
+        return flat_emit(pieces);
+    }
+    const int cut[3][4] = {{0, lo[0], hi[0], res[0]}, {0, lo[1], hi[1], res[1]}, {0, lo[2], hi[2], res[2]}};
+    for (int u = 0; u < 3; u++)
+        for (int v = 0; v < 3; v++)
+            for (int s = 0; s < 3; s++) {
+                if (u == 1 && v == 1 && s == 1) continue;
+                const int a[3] = {cut[0][u], cut[1][v], cut[2][s]}, b[3] = {cut[0][u + 1], cut[1][v + 1], cut[2][s + 1]};
+                box(a, b);
+            }
+    if (inner) {
+        const size_t n0 = pieces.size();
+        box(lo, hi);
+        for (size_t q = n0; q < pieces.size(); q++) pieces[q].flags |= FB_INNER;
+    }
+    // by plane, so that the pieces of a row run at about the same time; a box
+    // with few groups a plane keeps 8 blocks' worth of planes together
+    std::stable_sort(pieces.begin(), pieces.end(), [](const FlatBlock &x, const FlatBlock &y) { return x.i0 < y.i0; });
+    return flat_emit(pieces);
 }
 
 int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool pole_arrays)
@@ -671,7 +788,7 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
     // CPML
     for (int f = 0; f < 6; f++) {
         d.cp_on[f] = hp.cp[f].enabled;
-        d.cp_d[f] = hp.cp[f].depth;
+        d.cp_d[f] = hp.cp[f].enabled ? hp.cp[f].depth : 0;
         if (!hp.cp[f].enabled) continue;
         const int dep = hp.cp[f].depth;
         float *be, *ce, *bh, *ch;
@@ -939,68 +1056,78 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
         }
         if (f.nfreq > 0) bytes += (double)cell.size() * (9.0 * esz + (double)f.nfreq * 6 * 16 * 2);
     }
-    // work decomposition: the bulk box (outside every CPML slab, one extra
-    // plane on the low sides so that its halo row/column/plane is slab-free,
-    // off the grid's edge planes, k bounds multiples of 4) goes to the TMA
-    // kernel when the k rows are 16-byte multiples; the rest (slabs, edge
-    // planes) to the slab kernels
+    // work decomposition.  Large grids whose k rows are 16-byte multiples: the
+    // interior box (outside every CPML slab, one extra plane on the low sides
+    // so that its halo row/column/plane is slab-free, off the grid's edge
+    // planes, k bounds multiples of 4) goes to the TMA kernel and the rest
+    // (slabs, edge planes) to the flat kernels; else the flat kernels take all.
     {
         const int X = hp.xr, Y = hp.yr, Z = hp.zr;
         int lo[3], hi[3];
         const int res[3] = {X, Y, Z};
-        for (int ax = 0; ax < 3; ax++) {
-            lo[ax] = std::max(1, hp.cp[2 * ax].enabled ? hp.cp[2 * ax].depth + 1 : 0);
-            hi[ax] = std::min(res[ax] - 1, hp.cp[2 * ax + 1].enabled ? res[ax] - hp.cp[2 * ax + 1].depth : res[ax]);
-        }
-        lo[2] = std::max(4, (lo[2] + 3) / 4 * 4);   // the k halo group k0-4..k0-1 stays in the grid
-        hi[2] = hi[2] / 4 * 4;
         const char *nob = getenv("GSVIT_B200_NO_BULK");
-        // (design cells take the bulk kernel's per-cell coefficient path; those
-        // outside the box take e_special's)
-        P->bulk_on = !r64 && ((size_t)Z * esz % 16 == 0) && lo[0] < hi[0] && lo[1] < hi[1] && lo[2] < hi[2] && !(nob && nob[0] == '1');
-        std::vector<SlabBox> boxes;
+        const bool no_bulk = nob && nob[0] == '1';
+        P->fwidth = flat_width(P->storage, Z);
+        // The bulk kernel moves 49 bytes a cell, the flat pair 74, but its tiles
+        // want many planes: rough surface, us a step, flat alone / with the bulk
+        // kernel: 64^3 30 / 97, 128^3 85 / 128, 192^3 196 / 223, 256^3 393 / 402,
+        // 320^3 709 / 688, 384^3 1198 / 1090, 512^3 2699 / 2305.
+        // BF16 takes it wherever it can: it updates E from H before H is rounded,
+        // and stochastic rounding would carry that difference everywhere.
+        const double bulk_min = P->storage == FDTD_STORE_BF16 ? 0.0 : 25165824.0;
+        for (int pass = 0; pass < 2; pass++) {
+            P->bulk_on = pass == 0;   // first the TMA kernel's box, then the flat kernels' plain box
+            for (int ax = 0; ax < 3; ax++) {
+                const bool cl = hp.cp[2 * ax].enabled, ch = hp.cp[2 * ax + 1].enabled;
+                lo[ax] = std::max(1, cl ? hp.cp[2 * ax].depth + (P->bulk_on ? 1 : 0) : 0);
+                hi[ax] = std::min(res[ax] - 1, ch ? res[ax] - hp.cp[2 * ax + 1].depth : res[ax]);
+            }
+            const int ka = P->bulk_on ? 4 : P->fwidth;
+            if (P->bulk_on) lo[2] = std::max(4, lo[2]);   // the k halo group k0-4..k0-1 stays in the grid
+            lo[2] = (lo[2] + ka - 1) / ka * ka;
+            hi[2] = hi[2] / ka * ka;
+            // (design cells take per-cell coefficients in either kernel)
+            if (P->bulk_on && !r64 && (size_t)Z * esz % 16 == 0 && lo[0] < hi[0] && lo[1] < hi[1] && lo[2] < hi[2] && !no_bulk &&
+                (double)hp.n >= bulk_min)
+                break;
+        }
         std::vector<BulkItem> blk;
-        long long nblk = 0;
-        auto add_box = [&](int i0, int i1, int j0, int j1, int k0, int k1) {
-            if (i0 >= i1 || j0 >= j1 || k0 >= k1) return;
-            // TSF corrections touch cells in [t0 - 1, t1] on every axis (tsf_add_h/e)
-            const bool meets = d.tsf_on && i0 <= d.t1[0] && i1 >= d.t0[0] && j0 <= d.t1[1] && j1 >= d.t0[1] &&
-                               k0 <= d.t1[2] && k1 >= d.t0[2];
-            boxes.push_back({i0, i1, j0, j1, k0, k1, nblk, 0, meets ? 1 : 0});
-            nblk += ((long long)(i1 - i0) * (j1 - j0) * (k1 - k0) + 255) / 256;
-        };
         // planes per work item: about 10.  CTAs of neighbouring tiles then stay
         // within a few planes of each other, so that the halo rows and columns
         // one reads are still in L2 when the other reads them (the tiles of the
         // Drude-metal half run about 2x slower than the vacuum half: with 96
         // planes per item their drift evicted the halos; 512^3 rough surface,
         // bulk kernel 2.24 ms at 96 planes, 1.72 ms at 8-12, 1.79 ms at 4)
-        auto chunks = [&](int a0, int a1, int *len) {
-            const int planes = a1 - a0;
-            const int nch = std::max(1, (planes + 9) / 10);
-            *len = (planes + nch - 1) / nch;
-        };
         if (P->bulk_on) {
-            add_box(0, lo[0], 0, Y, 0, Z);
-            add_box(hi[0], X, 0, Y, 0, Z);
-            add_box(lo[0], hi[0], 0, lo[1], 0, Z);
-            add_box(lo[0], hi[0], hi[1], Y, 0, Z);
-            add_box(lo[0], hi[0], lo[1], hi[1], 0, lo[2]);
-            add_box(lo[0], hi[0], lo[1], hi[1], hi[2], Z);
-            int len;
-            chunks(lo[0], hi[0], &len);
+            const int planes = hi[0] - lo[0], nch = std::max(1, (planes + 9) / 10), len = (planes + nch - 1) / nch;
             blk = bulk_items(lo, hi, len, 0);
             P->bulk_len = len;
             for (int ax = 0; ax < 3; ax++) { P->region[2 * ax] = lo[ax]; P->region[2 * ax + 1] = hi[ax]; }
-        } else {
-            add_box(0, X, 0, Y, 0, Z);
         }
-        if (nblk > 0x7fffffffLL) return bail(cudaErrorInvalidValue, "grid too large for the slab kernels");
-        {   // algorithmic bytes per launch: 24 B field reads + 24 B writes + 1 class byte per cell;
-            // 12 B (Q read + write, E^{n-1} read) + 16 B per pole per dispersive field component;
-            // 4 psi arrays x (4 B read + 4 B write) per CPML cell (slab kernels only)
+        if ((double)hp.n / P->fwidth / FLAT_NT > 1.0e9) return bail(cudaErrorInvalidValue, "grid too large for the flat kernels");
+        P->h_flat = flat_blocks(hp, d, lo, hi, !P->bulk_on, P->fwidth);
+        std::vector<FlatBlock> part[2];   // the rest, the interior
+        for (const FlatBlock &b : P->h_flat) part[(b.flags & FB_INNER) != 0].push_back(b);
+        const bool inner = P->bulk_on || !part[1].empty();
+        {
+            auto list = [&](const std::vector<FlatBlock> &v, FlatList *l) {
+                FlatBlock *dv = nullptr;
+                l->n = (unsigned)v.size();
+                if (v.empty()) return cudaSuccess;
+                cudaError_t e = upload(P->mem, &dv, v.data(), v.size());
+                l->blocks = dv;
+                return e;
+            };
+            CA(list(P->h_flat, &P->flat), "flat blocks");
+            CA(list(part[0], &P->flat_sp), "flat blocks");
+            CA(list(part[1], &P->flat_in), "flat blocks");
+        }
+        {   // algorithmic bytes per step of the interior and of the rest: 24 B field reads + 24 B writes
+            // + 1 class byte per cell; 12 B (Q read + write, E^{n-1} read) + 16 B per pole per dispersive
+            // field component; 4 psi arrays x (4 B read + 4 B write) per CPML cell (the rest only)
             auto cell_bytes = [&](int i0, int i1, int j0, int j1, int k0, int k1) {
                 double b = 0;
+                if (i0 >= i1 || j0 >= j1 || k0 >= k1) return b;
 #pragma omp parallel for reduction(+ : b) schedule(static)
                 for (int i = i0; i < i1; i++)
                     for (int j = j0; j < j1; j++)
@@ -1013,99 +1140,14 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
                         }
                 return b;
             };
-            double total = 0;
-            for (auto &b : boxes) total += cell_bytes(b.i0, b.i1, b.j0, b.j1, b.k0, b.k1);
             double psi = 0;
             for (int f = 0; f < 6; f++)
                 if (hp.cp[f].enabled) {
                     const int dep = hp.cp[f].depth;
                     psi += ((f < 2) ? (double)dep * Y * Z : (f < 4) ? (double)X * dep * Z : (double)X * Y * dep) * 4 * 2.0 * esz;
                 }
-            P->slab_bytes = total + psi;
-            P->bulk_bytes = P->bulk_on ? cell_bytes(lo[0], hi[0], lo[1], hi[1], lo[2], hi[2]) : 0;
-        }
-        CA(upload(P->mem, &P->d_boxes, boxes.data(), boxes.size()), "slab boxes");
-        {   // 4-cell groups for the H kernel when every box's k bounds and the row length allow
-            bool w4 = (Z % 4 == 0);
-            for (auto &b : boxes) w4 = w4 && b.k0 % 4 == 0 && b.k1 % 4 == 0;
-            if (w4 && !boxes.empty()) {
-                std::vector<SlabBox> b4 = boxes;
-                long long nb = 0;
-                for (auto &b : b4) {
-                    b.first_block = nb;
-                    nb += ((long long)(b.i1 - b.i0) * (b.j1 - b.j0) * ((b.k1 - b.k0) / 4) + 255) / 256;
-                }
-                CA(upload(P->mem, &P->d_boxes4, b4.data(), b4.size()), "slab boxes");
-                P->nslab_blocks4 = nb;
-            }
-        }
-        P->h_boxes = boxes;
-        P->h_bulk = blk;
-        P->nboxes = (int)boxes.size();
-        P->nslab_blocks = nblk;
-        {   // E lists: each box split along k into runs of planes that hold a
-            // dispersive cell and runs that hold none; plain runs shorter than
-            // 8 planes stay with the dispersive list (its kernel handles plain
-            // cells the same way), so the split adds few boxes
-            std::vector<SlabBox> eb, pb;
-            long long neb = 0, npb = 0;
-            auto push = [&](const SlabBox &b0, int k0, int k1, bool disp) {
-                SlabBox b = b0;
-                b.k0 = k0;
-                b.k1 = k1;
-                long long &n = disp ? neb : npb;
-                b.first_block = n;
-                n += ((long long)(b.i1 - b.i0) * (b.j1 - b.j0) * (k1 - k0) + 255) / 256;
-                (disp ? eb : pb).push_back(b);
-            };
-            for (const SlabBox &b : boxes) {
-                if (!hp.has_ade) { push(b, b.k0, b.k1, true); continue; }
-                std::vector<char> dk(b.k1 - b.k0, 0);
-#pragma omp parallel for schedule(static)
-                for (int k = b.k0; k < b.k1; k++) {
-                    char any = 0;
-                    for (int i = b.i0; i < b.i1 && !any; i++)
-                        for (int j = b.j0; j < b.j1; j++)
-                            if (hp.classes[hp.cls[((size_t)i * Y + j) * Z + k]].flags & CF_ADE_BRANCH) { any = 1; break; }
-                    dk[k - b.k0] = any;
-                }
-                for (int k = b.k0; k < b.k1;) {   // short plain runs count as dispersive
-                    int e = k;
-                    while (e < b.k1 && dk[e - b.k0] == dk[k - b.k0]) e++;
-                    if (!dk[k - b.k0] && e - k < 8)
-                        for (int q = k; q < e; q++) dk[q - b.k0] = 1;
-                    k = e;
-                }
-                for (int k = b.k0; k < b.k1;) {
-                    int e = k;
-                    while (e < b.k1 && dk[e - b.k0] == dk[k - b.k0]) e++;
-                    push(b, k, e, dk[k - b.k0] != 0);
-                    k = e;
-                }
-            }
-            P->h_eboxes = pb.empty() ? boxes : eb;
-            P->h_epboxes = pb;
-            SlabLists &L = P->slabs;
-            L.h = P->d_boxes;
-            L.nh = P->nboxes;
-            L.hblocks = nblk;
-            L.h4 = P->d_boxes4;
-            L.h4blocks = P->nslab_blocks4;
-            if (pb.empty()) {
-                L.e = P->d_boxes;
-                L.ne = P->nboxes;
-                L.eblocks = nblk;
-            } else {
-                SlabBox *de = nullptr, *dp = nullptr;
-                if (!eb.empty()) CA(upload(P->mem, &de, eb.data(), eb.size()), "slab boxes");
-                CA(upload(P->mem, &dp, pb.data(), pb.size()), "slab boxes");
-                L.e = de;
-                L.ne = (int)eb.size();
-                L.eblocks = neb;
-                L.ep = dp;
-                L.nep = (int)pb.size();
-                L.epblocks = npb;
-            }
+            P->bulk_bytes = inner ? cell_bytes(lo[0], hi[0], lo[1], hi[1], lo[2], hi[2]) : 0;
+            P->slab_bytes = cell_bytes(0, X, 0, Y, 0, Z) - P->bulk_bytes + psi;
         }
         CA(P->mem.alloc(&P->d_err, 1), "error word");
         if (P->bulk_on) {
@@ -1133,16 +1175,17 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
                 if (hp.cp[f].enabled) dmin = std::min(dmin, hp.cp[f].depth);
         }
         const bool can_tile = !r64 && roomy && ((size_t)Z * esz % 16 == 0) && !(nob && nob[0] == '1');
-        // Default: tiles for grids of at least 2^24 cells with CPML of depth
-        // >= 12.  Rough-surface steps, ms, slab kernels / tiles (the CPML kinds
-        // concurrent with the bulk): 512^3 d16 3.11 / 2.74, 384^3 d16 1.56 /
-        // 1.39, 256^3 d16 0.62 / 0.58, 256^3 d12 0.59 / 0.59; smaller grids
-        // and thinner slabs fill the CPML tiles poorly and the slab kernels
-        // win: 256x256x128 d12 0.42 / 0.44, 192^3 d16 0.36 / 0.40, 128^3 d8
-        // 0.16 / 0.21.  GSVIT_B200_TILES=1 / 0 at plan creation forces them
-        // on / off.
+        // which order the faces of a corner cell come in: a matter of rounding
+        // alone, kept as the CPML tiles had it where they used to run
+        const bool tile_size = dmin >= 12 && (double)hp.n >= 16777216.0;
+        d.axis_order = can_tile && tile_size;
+        // The CPML tiles run for large BF16 grids (as the bulk kernel above) and on
+        // request (GSVIT_B200_TILES=1 at plan creation; 0 forces them off): the flat
+        // kernels, beside the bulk kernel or alone, are faster at every size
+        // (rough surface, ms a step, tiles / bulk and flat: 512^3 d16 2.65 / 2.31,
+        // 256^3 d16 0.55 / 0.39, 192^3 d16 0.35 / 0.20, 64^3 d8 0.139 / 0.030).
         const char *tv = getenv("GSVIT_B200_TILES");
-        const bool want = tv ? tv[0] == '1' : (dmin >= 12 && (double)hp.n >= 16777216.0);
+        const bool want = tv ? tv[0] == '1' : P->storage == FDTD_STORE_BF16 && tile_size;
         P->tiles_on = can_tile && want;
         // test hook of the bounded-wait error path: every tile CTA of this plan
         // also waits, at most this many polls, on an mbarrier nothing arrives on
@@ -1151,7 +1194,7 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
             int rc = build_tiles(P, hp, d, cls);
             if (rc != FDTD_OK) return bail_rc(rc);
         }
-        if (P->tiles_on || P->bulk_on) {   // side streams and events of the concurrent CPML kinds / slab H
+        if (P->tiles_on || P->bulk_on) {   // side streams and events of the concurrent CPML kinds / flat H
             CA(cudaEventCreateWithFlags(&P->ev_fork, cudaEventDisableTiming), "tile events");
             for (int k = TILE_CPX; k < NTILE; k++) {
                 CA(cudaStreamCreateWithFlags(&P->side[k], cudaStreamNonBlocking), "tile streams");
@@ -1590,14 +1633,17 @@ int fdtd_step_profile(fdtd_plan *P, int nsteps, double out[8])
             for (int kind = TILE_CPX; kind < NTILE && rc == FDTD_OK; kind++) rc = launch_tile_kind(P, d, in, kind, st);
             if (rc != FDTD_OK) return rc;
         } else {
-            if (P->bulk_on) {
-                cudaError_t e = launch_tiles(TILE_BULK, d, P->bmaps[in], P->d_bulk, P->nbulk, P->d_err, P->hp.has_ade,
-                                             P->hp.maxpoles, P->storage, 0, st);
-                if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("bulk step launch: ") + cudaGetErrorString(e));
-            }
+            // the boxes around the interior (H), the interior, those boxes (E)
+            cudaError_t e = launch_flat_h(d, P->flat_sp, P->fwidth, P->storage, st);
+            CK(cudaEventRecord(E[5], st));
+            if (e == cudaSuccess && P->bulk_on)
+                e = launch_tiles(TILE_BULK, d, P->bmaps[in], P->d_bulk, P->nbulk, P->d_err, P->hp.has_ade, P->hp.maxpoles,
+                                 P->storage, 0, st);
+            if (e == cudaSuccess) e = launch_flat_h(d, P->flat_in, P->fwidth, P->storage, st);
+            if (e == cudaSuccess) e = launch_flat_e(d, P->flat_in, P->fwidth, P->hp.has_ade, P->hp.maxpoles, P->storage, st);
             CK(cudaEventRecord(E[2], st));
-            cudaError_t e = launch_slab_steps(d, P->slabs, P->hp.has_ade, P->hp.maxpoles, P->storage, st);
-            if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("slab step launch: ") + cudaGetErrorString(e));
+            if (e == cudaSuccess) e = launch_flat_e(d, P->flat_sp, P->fwidth, P->hp.has_ade, P->hp.maxpoles, P->storage, st);
+            if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("flat step launch: ") + cudaGetErrorString(e));
         }
         CK(cudaEventRecord(E[3], st));
         launch_nfff(P, in, st);
@@ -1616,6 +1662,12 @@ int fdtd_step_profile(fdtd_plan *P, int nsteps, double out[8])
         CK(cudaEventElapsedTime(&t23, E[2], E[3]));
         CK(cudaEventElapsedTime(&t34, E[3], E[4]));
         CK(cudaEventElapsedTime(&t04, E[0], E[4]));
+        if (!P->tiles_on) {   // E[1] .. E[5]: H of the boxes around the interior
+            float t15;
+            CK(cudaEventElapsedTime(&t15, E[1], E[5]));
+            t12 -= t15;
+            t23 += t15;
+        }
         aux += t01; bulk += t12; slab += t23; nf += t34; tot += t04;
     }
     for (auto &e : ev) cudaEventDestroy(e);
@@ -1633,8 +1685,7 @@ int fdtd_step_profile(fdtd_plan *P, int nsteps, double out[8])
     } else {
         out[1] = P->bulk_bytes;
         out[3] = P->slab_bytes;
-        const SlabLists &L = P->slabs;   // slab H, then E over the dispersive and the plain runs
-        nyee = (P->bulk_on ? 1 : 0) + (L.hblocks > 0 ? 1 + (L.eblocks > 0 ? 1 : 0) + (L.epblocks > 0 ? 1 : 0) : 0);
+        nyee = (P->bulk_on ? 1 : 0) + (P->flat.n > 0 ? 2 : 0);   // flat H, flat E
     }
     out[7] = 1 + (P->tsf_cells ? 1 : 0) + nyee + (P->nfff_nfreq > 0 ? 2 : 0) + (P->nfff_series ? 1 : 0);
     return FDTD_OK;
@@ -1799,24 +1850,16 @@ struct fdtd_batch {
     size_t items_cap[3] = {0, 0, 0};
     int nitems[3] = {0, 0, 0}, bulk_grid[3] = {0, 0, 0}, chunk_len = 0;
     bool persistent = true;
-    SlabBox *d_boxes[3] = {nullptr, nullptr, nullptr};
-    SlabBox *d_boxes4[3] = {nullptr, nullptr, nullptr};   // 4-cell groups when every box of the group is 4-aligned
-    int nboxes[3] = {0, 0, 0};
-    long long nslab_blocks[3] = {0, 0, 0};
-    long long nslab_blocks4[3] = {0, 0, 0};
-    SlabBox *d_eboxes[3] = {nullptr, nullptr, nullptr};   // E: the instances' dispersive runs, per variant
-    int neboxes[3] = {0, 0, 0};
-    long long neblocks[3] = {0, 0, 0};
-    SlabBox *d_epboxes = nullptr;                         // E: every instance's plain runs, one launch
-    int nepboxes = 0;
-    long long nepblocks = 0;
+    FlatList fh[2];          // H blocks of the instances, by cells per thread (a whole vector, one)
+    FlatList fe[3][2];       // E blocks, by variant group and cells per thread
+    int width[2] = {4, 1};
     int max_tsf = 0, max_nfff = 0;
     int *d_err = nullptr;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     int graph_steps = 0;
     // Each instance runs the path it runs alone: the TMA tiles over its whole
     // grid (fdtd_plan::tiles_on; their lists concatenated per kernel variant
-    // and tile kind, one CTA per item) or the bulk box and slab kernels (the
+    // and tile kind, one CTA per item) or the bulk box and flat kernels (the
     // lists above hold only these instances).
     int ntiled = 0;
     BulkItem *d_titems[3][NTILE] = {};   // [variant group][tile kind]
@@ -1885,25 +1928,17 @@ int batch_launch_step(fdtd_batch *B, cudaStream_t st)
                                                B->ntitems[g][kind], B->ncls, B->d_err, g > 0, g == 2 ? 2 : 0, B->storage, st);
             if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("batched tile launch: ") + cudaGetErrorString(e));
         }
-    // the others: bulk box and slab kernels, variant by variant (a side
-    // stream for the slab H kernels, as single plans have, measured slower on
-    // the 48-instance batch: 11.3 against 13.9 Gcell/s)
-    for (int g = 0; g < 3; g++) {
-        if (!B->nitems[g] && !B->nboxes[g] && !B->neboxes[g]) continue;
-        const bool ade = g > 0;
-        const int npoles = g == 2 ? 2 : 0;
-        cudaError_t e = launch_bulk_batch(B->d_plans[in], B->d_maps[in], B->d_items[g], B->nitems[g], B->bulk_grid[g], B->ncls,
-                                          B->d_err, ade, npoles, B->storage, st);
-        if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("batched bulk launch: ") + cudaGetErrorString(e));
-        e = launch_slab_steps_batch(B->d_plans[in], B->d_boxes[g], B->nboxes[g], B->nslab_blocks[g], B->d_boxes4[g],
-                                    B->nslab_blocks4[g], B->d_eboxes[g], B->neboxes[g], B->neblocks[g], ade, npoles,
-                                    B->storage, st);
-        if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("batched slab launch: ") + cudaGetErrorString(e));
-    }
-    if (B->nepboxes) {   // E of every instance's plain runs (after all H half steps)
-        cudaError_t e = launch_slab_e_plain_batch(B->d_plans[in], B->d_epboxes, B->nepboxes, B->nepblocks, B->storage, st);
-        if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("batched slab launch: ") + cudaGetErrorString(e));
-    }
+    // the others: flat H of every instance, the bulk boxes variant by variant
+    // (disjoint cells; both read the input set only), then flat E
+    cudaError_t e = cudaSuccess;
+    for (int w = 0; w < 2 && e == cudaSuccess; w++) e = launch_flat_h_batch(B->d_plans[in], B->fh[w], B->width[w], B->storage, st);
+    for (int g = 0; g < 3 && e == cudaSuccess; g++)
+        e = launch_bulk_batch(B->d_plans[in], B->d_maps[in], B->d_items[g], B->nitems[g], B->bulk_grid[g], B->ncls, B->d_err,
+                              g > 0, g == 2 ? 2 : 0, B->storage, st);
+    for (int g = 0; g < 3; g++)
+        for (int w = 0; w < 2 && e == cudaSuccess; w++)
+            e = launch_flat_e_batch(B->d_plans[in], B->fe[g][w], B->width[w], g > 0, g == 2 ? 2 : 0, B->storage, st);
+    if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("batched step launch: ") + cudaGetErrorString(e));
     if (B->max_nfff) launch_nfff_accumulate_batch(B->d_nfff[in], n, B->max_nfff, st);
     B->cur = 1 - in;
     return FDTD_OK;
@@ -1987,59 +2022,28 @@ int fdtd_batch_create(const fdtd_desc *descs, int nplans, int device, fdtd_batch
         BA(upload(B->mem, &B->d_aux[in], ax.data(), ax.size()), "batch tables");
         BA(upload(B->mem, &B->d_nfff[in], nf.data(), nf.size()), "batch tables");
     }
-    // slab boxes of every instance (numbered one cell per thread), per kernel variant
-    for (int g = 0; g < 3; g++) {
-        std::vector<SlabBox> boxes;
-        for (int q = 0; q < nplans; q++) {
-            if (B->group[q] != g || B->plans[q]->tiles_on) continue;
-            for (SlabBox b : B->plans[q]->h_boxes) {
-                b.first_block = B->nslab_blocks[g];
-                b.inst = q;
-                boxes.push_back(b);
-                B->nslab_blocks[g] += ((long long)(b.i1 - b.i0) * (b.j1 - b.j0) * (b.k1 - b.k0) + 255) / 256;
+    // flat boxes of every instance without TMA tiles
+    for (int w = 0; w < 2; w++) {
+        auto list = [&](int g, FlatList *l) {
+            std::vector<FlatBlock> v;
+            for (int q = 0; q < nplans; q++) {
+                const fdtd_plan *P = B->plans[q];
+                if (P->tiles_on || (P->fwidth == 1) != (w == 1) || (g >= 0 && B->group[q] != g)) continue;
+                for (FlatBlock b : P->h_flat) {
+                    b.inst = q;
+                    v.push_back(b);
+                }
             }
-        }
-        if (B->nslab_blocks[g] > 0x7fffffffLL) { fail(FDTD_E_UNSUPPORTED, "too many slab cells for one launch"); return bail(FDTD_E_UNSUPPORTED); }
-        BA(upload(B->mem, &B->d_boxes[g], boxes.data(), boxes.size()), "batch slab boxes");
-        B->nboxes[g] = (int)boxes.size();
-        // E runs with a dispersive cell, numbered for this variant's launch
-        std::vector<SlabBox> ebx;
-        for (int q = 0; q < nplans; q++) {
-            if (B->group[q] != g || B->plans[q]->tiles_on) continue;
-            for (SlabBox b : B->plans[q]->h_eboxes) {
-                b.first_block = B->neblocks[g];
-                b.inst = q;
-                ebx.push_back(b);
-                B->neblocks[g] += ((long long)(b.i1 - b.i0) * (b.j1 - b.j0) * (b.k1 - b.k0) + 255) / 256;
-            }
-        }
-        if (B->neblocks[g] > 0x7fffffffLL) { fail(FDTD_E_UNSUPPORTED, "too many slab cells for one launch"); return bail(FDTD_E_UNSUPPORTED); }
-        if (!ebx.empty()) BA(upload(B->mem, &B->d_eboxes[g], ebx.data(), ebx.size()), "batch slab boxes");
-        B->neboxes[g] = (int)ebx.size();
-        bool w4 = !boxes.empty();
-        for (auto &b : boxes) w4 = w4 && B->plans[b.inst]->hp.zr % 4 == 0 && b.k0 % 4 == 0 && b.k1 % 4 == 0;
-        if (w4) {
-            for (auto &b : boxes) {
-                b.first_block = B->nslab_blocks4[g];
-                B->nslab_blocks4[g] += ((long long)(b.i1 - b.i0) * (b.j1 - b.j0) * ((b.k1 - b.k0) / 4) + 255) / 256;
-            }
-            BA(upload(B->mem, &B->d_boxes4[g], boxes.data(), boxes.size()), "batch slab boxes");
-        }
-    }
-    {   // E runs without a dispersive cell, every instance in one launch
-        std::vector<SlabBox> pbx;
-        for (int q = 0; q < nplans; q++) {
-            if (B->plans[q]->tiles_on) continue;
-            for (SlabBox b : B->plans[q]->h_epboxes) {
-                b.first_block = B->nepblocks;
-                b.inst = q;
-                pbx.push_back(b);
-                B->nepblocks += ((long long)(b.i1 - b.i0) * (b.j1 - b.j0) * (b.k1 - b.k0) + 255) / 256;
-            }
-        }
-        if (B->nepblocks > 0x7fffffffLL) { fail(FDTD_E_UNSUPPORTED, "too many slab cells for one launch"); return bail(FDTD_E_UNSUPPORTED); }
-        if (!pbx.empty()) BA(upload(B->mem, &B->d_epboxes, pbx.data(), pbx.size()), "batch slab boxes");
-        B->nepboxes = (int)pbx.size();
+            if (v.size() > 0x7fffffffu) return cudaErrorInvalidConfiguration;
+            l->n = (unsigned)v.size();
+            if (v.empty()) return cudaSuccess;
+            FlatBlock *dv = nullptr;
+            cudaError_t e = upload(B->mem, &dv, v.data(), v.size());
+            l->blocks = dv;
+            return e;
+        };
+        BA(list(-1, &B->fh[w]), "batch flat blocks");
+        for (int g = 0; g < 3; g++) BA(list(g, &B->fe[g][w]), "batch flat blocks");
     }
     BA(B->mem.alloc(&B->d_err, 1), "error word");
     for (auto *P : B->plans) P->batch_err = B->d_err;   // the instances' readbacks check the batch's word too

@@ -41,7 +41,6 @@
 
 #include "fdtd_bulk.cuh"
 #include "../../include/gsvit_b200.h"
-#include "fdtd_cells.cuh"
 #include "fdtd_cpgroup.cuh"
 #include "fdtd_device.cuh"
 
@@ -369,10 +368,7 @@ __device__ __forceinline__ bool bulk_item(const DevPlan &P, const BulkMaps &M, c
                     hy[c] = da[c] * hy[c] + db[c] * ((ezi[c] - ez[c]) - (exk - ex[c]));
                     hz[c] = da[c] * hz[c] + db[c] * ((exj[c] - ex[c]) - (eyi[c] - ey[c]));
                 }
-                if (tsf_plane) {
-#pragma unroll
-                    for (int c = 0; c < 4; c++) tsf_add_h(P, i, j, kq + c, hx[c], hy[c], hz[c]);
-                }
+                if (tsf_plane) tsf_add_h<float, 4>(P, i, j, kq, hx, hy, hz);
             } else if (special) {
                 // ystep_h with kappa and the edge rules, then psi_H, TSF and the
                 // zeroed planes (fdtd_cpgroup.cuh); psi_H is written by the owner
@@ -529,10 +525,7 @@ __device__ __forceinline__ bool bulk_item(const DevPlan &P, const BulkMaps &M, c
                         if (fl & CF_PEC_Z) ne[2][c] = 0.f;
                     }
                 }
-                if (tsf_plane) {
-#pragma unroll
-                    for (int c = 0; c < 4; c++) tsf_add_e(P, i, j, kq + c, ne[0][c], ne[1][c], ne[2][c]);
-                }
+                if (tsf_plane) tsf_add_e<float, 4>(P, i, j, kq, ne[0], ne[1], ne[2]);
                 if (ADE) {
 #pragma unroll
                     for (int a = 0; a < 3; a++) {

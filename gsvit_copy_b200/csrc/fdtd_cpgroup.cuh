@@ -27,7 +27,6 @@
 #include <cuda_runtime.h>
 
 #include "fdtd_bulk.cuh"
-#include "fdtd_cells.cuh"
 #include "fdtd_device.cuh"
 
 namespace {
@@ -121,9 +120,9 @@ __device__ __forceinline__ void cp_h_group(const DevPlan &P, const float4 *scls,
         if (!(jl || kl)) hx[c] = da * hx[c] + db * (dey_k[c] * ikz - dez_j[c] * iky);
         if (!(il || kl)) hy[c] = da * hy[c] + db * (dez_i[c] * ikx - dex_k[c] * ikz);
         if (!(il || jl)) hz[c] = da * hz[c] + db * (dex_j[c] * iky - dey_i[c] * ikx);
-        if (tsf && P.tsf_on) tsf_add_h(P, i, j, k, hx[c], hy[c], hz[c]);
         dbdx[c] = db * dx;
     }
+    if (tsf && P.tsf_on) tsf_add_h<float, 4>(P, i, j, kq, hx, hy, hz);
     const bool kall = kin[0] && kin[1] && kin[2] && kin[3];
     // x faces: psi[1] <- dey_i (hz -= dbdx psi), psi[0] <- dez_i (hy += dbdx psi)
     auto xface = [&](int f, int pos) {
@@ -498,10 +497,9 @@ __device__ __forceinline__ void cp_e_group(const DevPlan &P, const float4 *scls,
         }
     }
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
+    for (int c = 0; c < 4; c++)
         if (zero[c]) ne[0][c] = ne[1][c] = ne[2][c] = 0.f;
-        if (tsf && P.tsf_on) tsf_add_e(P, i, j, kq + c, ne[0][c], ne[1][c], ne[2][c]);
-    }
+    if (tsf && P.tsf_on) tsf_add_e<float, 4>(P, i, j, kq, ne[0], ne[1], ne[2]);
 }
 
 }  // namespace

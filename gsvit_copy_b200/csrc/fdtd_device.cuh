@@ -8,6 +8,9 @@
 
 #include "fdtd_internal.h"
 
+// faces of the grid
+enum { X0 = 0, XN = 1, Y0 = 2, YN = 3, Z0 = 4, ZN = 5 };
+
 // ---- field storage: FP32, FP16, BF16 or FP64 elements behind the float
 // pointers of DevPlan.  Arithmetic is FP32 (Stor<T>::real) for the first three
 // and FP64 for FP64 storage (the reference-precision mode).  Stor<T>::scaled
@@ -384,51 +387,74 @@ __device__ __forceinline__ double tsf_dval(const double *data, int res, double x
     return 0;
 }
 
-// Add the precomputed TSF corrections of this step to the H cell (i,j,k).
-// Face order as the reference applies them: i0, in, j0, jn, k0, kn
+// Add the precomputed TSF corrections of this step to the H cells (i, j, k ..
+// k+V-1).  Face order as the reference applies them: i0, in, j0, jn, k0, kn
 // (source.c:1476-1672); components (hy,hz) on i faces, (hx,hz) on j faces,
-// (hx,hy) on k faces.
-template <class R>
-__device__ __forceinline__ void tsf_add_h(const DevPlan &P, int i, int j, int k, R &hx, R &hy, R &hz)
+// (hx,hy) on k faces.  A k face meets one cell of the group: its correction is
+// read once and added under a per-cell predicate, since nearly every warp
+// that covers whole k rows holds such a group.
+template <class R, int V>
+__device__ __forceinline__ void tsf_face_rows(const typename Tab<R>::V2 *row, int off, R (&a)[V], R (&b)[V], int n)
+{
+#pragma unroll
+    for (int c = 0; c < V; c++) {
+        if (off + c < 0 || off + c > n) continue;
+        const auto d = row[off + c];
+        a[c] += d.x;
+        b[c] += d.y;
+    }
+}
+template <class R, int V>
+__device__ __forceinline__ void tsf_face_cell_add(const typename Tab<R>::V2 *p, int at, R (&a)[V], R (&b)[V])
+{
+    const auto d = *p;
+#pragma unroll
+    for (int c = 0; c < V; c++)
+        if (c == at) { a[c] += d.x; b[c] += d.y; }
+}
+template <class R, int V>
+__device__ __forceinline__ void tsf_add_h(const DevPlan &P, int i, int j, int k, R (&hx)[V], R (&hy)[V], R (&hz)[V])
 {
     using V2 = typename Tab<R>::V2;
     const V2 *const *tc = reinterpret_cast<const V2 *const *>(P.tcor_h);
     const int i0 = P.t0[0], j0 = P.t0[1], k0 = P.t0[2], in = P.t1[0], jn = P.t1[1], kn = P.t1[2];
-    const bool ji = j >= j0 && j <= jn, ki = k >= k0 && k <= kn, ii = i >= i0 && i <= in;
-    if (ji && ki) {
-        if (i == i0 - 1) { const V2 d = tc[0][(j - j0) * P.tnb[0] + (k - k0)]; hy += d.x; hz += d.y; }
-        if (i == in) { const V2 d = tc[1][(j - j0) * P.tnb[1] + (k - k0)]; hy += d.x; hz += d.y; }
+    const bool ji = j >= j0 && j <= jn, ii = i >= i0 && i <= in;
+    if (ji) {
+        if (i == i0 - 1) tsf_face_rows<R, V>(tc[0] + (j - j0) * P.tnb[0], k - k0, hy, hz, kn - k0);
+        if (i == in) tsf_face_rows<R, V>(tc[1] + (j - j0) * P.tnb[1], k - k0, hy, hz, kn - k0);
     }
-    if (ii && ki) {
-        if (j == j0 - 1) { const V2 d = tc[2][(i - i0) * P.tnb[2] + (k - k0)]; hx += d.x; hz += d.y; }
-        if (j == jn) { const V2 d = tc[3][(i - i0) * P.tnb[3] + (k - k0)]; hx += d.x; hz += d.y; }
-    }
-    if (ii && ji) {
-        if (k == k0 - 1) { const V2 d = tc[4][(i - i0) * P.tnb[4] + (j - j0)]; hx += d.x; hy += d.y; }
-        if (k == kn) { const V2 d = tc[5][(i - i0) * P.tnb[5] + (j - j0)]; hx += d.x; hy += d.y; }
+    if (ii) {
+        if (j == j0 - 1) tsf_face_rows<R, V>(tc[2] + (i - i0) * P.tnb[2], k - k0, hx, hz, kn - k0);
+        if (j == jn) tsf_face_rows<R, V>(tc[3] + (i - i0) * P.tnb[3], k - k0, hx, hz, kn - k0);
+        if (ji) {
+            const int q = k0 - 1 - k, r = kn - k;
+            if (q >= 0 && q < V) tsf_face_cell_add<R, V>(tc[4] + (i - i0) * P.tnb[4] + (j - j0), q, hx, hy);
+            if (r >= 0 && r < V) tsf_face_cell_add<R, V>(tc[5] + (i - i0) * P.tnb[5] + (j - j0), r, hx, hy);
+        }
     }
 }
 
-// Same for the E cell (source.c:547-771): (ey,ez) on i faces, (ex,ez) on j
+// Same for the E cells (source.c:547-771): (ey,ez) on i faces, (ex,ez) on j
 // faces, (ex,ey) on k faces.
-template <class R>
-__device__ __forceinline__ void tsf_add_e(const DevPlan &P, int i, int j, int k, R &ex, R &ey, R &ez)
+template <class R, int V>
+__device__ __forceinline__ void tsf_add_e(const DevPlan &P, int i, int j, int k, R (&ex)[V], R (&ey)[V], R (&ez)[V])
 {
     using V2 = typename Tab<R>::V2;
     const V2 *const *tc = reinterpret_cast<const V2 *const *>(P.tcor_e);
     const int i0 = P.t0[0], j0 = P.t0[1], k0 = P.t0[2], in = P.t1[0], jn = P.t1[1], kn = P.t1[2];
-    const bool ji = j >= j0 && j <= jn, ki = k >= k0 && k <= kn, ii = i >= i0 && i <= in;
-    if (ji && ki) {
-        if (i == i0) { const V2 d = tc[0][(j - j0) * P.tnb[0] + (k - k0)]; ey += d.x; ez += d.y; }
-        if (i == in) { const V2 d = tc[1][(j - j0) * P.tnb[1] + (k - k0)]; ey += d.x; ez += d.y; }
+    const bool ji = j >= j0 && j <= jn, ii = i >= i0 && i <= in;
+    if (ji) {
+        if (i == i0) tsf_face_rows<R, V>(tc[0] + (j - j0) * P.tnb[0], k - k0, ey, ez, kn - k0);
+        if (i == in) tsf_face_rows<R, V>(tc[1] + (j - j0) * P.tnb[1], k - k0, ey, ez, kn - k0);
     }
-    if (ii && ki) {
-        if (j == j0) { const V2 d = tc[2][(i - i0) * P.tnb[2] + (k - k0)]; ex += d.x; ez += d.y; }
-        if (j == jn) { const V2 d = tc[3][(i - i0) * P.tnb[3] + (k - k0)]; ex += d.x; ez += d.y; }
-    }
-    if (ii && ji) {
-        if (k == k0) { const V2 d = tc[4][(i - i0) * P.tnb[4] + (j - j0)]; ex += d.x; ey += d.y; }
-        if (k == kn) { const V2 d = tc[5][(i - i0) * P.tnb[5] + (j - j0)]; ex += d.x; ey += d.y; }
+    if (ii) {
+        if (j == j0) tsf_face_rows<R, V>(tc[2] + (i - i0) * P.tnb[2], k - k0, ex, ez, kn - k0);
+        if (j == jn) tsf_face_rows<R, V>(tc[3] + (i - i0) * P.tnb[3], k - k0, ex, ez, kn - k0);
+        if (ji) {
+            const int q = k0 - k, r = kn - k;
+            if (q >= 0 && q < V) tsf_face_cell_add<R, V>(tc[4] + (i - i0) * P.tnb[4] + (j - j0), q, ex, ey);
+            if (r >= 0 && r < V) tsf_face_cell_add<R, V>(tc[5] + (i - i0) * P.tnb[5] + (j - j0), r, ex, ey);
+        }
     }
 }
 

@@ -1,0 +1,4 @@
+// fdtd_flat_f32.cu -- the flat step kernels of one storage type.
+#include "fdtd_flat_kernels.cuh"
+
+FLAT_INSTANCE(float)

@@ -124,7 +124,8 @@ struct DevPlan {
     float *q[3];                    // Drude current Q per component
     float *pc[3][2], *qc[3][2];     // critical-point poles: p and q per component
     // CPML: face order x0 xn y0 yn z0 zn
-    int cp_on[6], cp_d[6];
+    int cp_on[6], cp_d[6];          // cp_d 0 for a face without CPML
+    int axis_order;                 // corner cells take their faces axis by axis (x, y, z), else x0 y0 z0 xn yn zn
     const float *be[6], *ce[6], *bh[6], *ch[6];
     const float *ike[3], *ikh[3];   // 1/kappa per axis (E and H), length xr / yr / zr
     float *psie[6][2];              // x: {peyx, pezx} y: {pexy, pezy} z: {pexz, peyz}

@@ -1,223 +1,15 @@
-// fdtd_kernels.cu -- sm_100a kernels of one GSvit FDTD time step.
-//
-// One step = aux_step (1D TSF grid, 1 CTA) -> bulk kernel (fdtd_bulk.cu,
-// fused H+E over the slab-free box) -> slab H -> slab E (the CPML slabs and
-// grid edges left outside the bulk box) -> nfff_accumulate (running DFT).
-//
-// The slab kernels walk a list of boxes (SlabBox) with a flat block index.
-// slab_h_kernel updates one cell per thread: ystep_h (yee.c:146-265), then
-// h_special -- the CPML psi_H update and corrections (boundary.c:347-519),
-// the TSF H corrections (source.c:1464-1672) and the zeroed outer planes.
-// slab_h4_kernel is the same update on four consecutive k cells per thread
-// with 16-byte loads, used when every box is 4-aligned in k.  slab_e_kernel
-// updates one cell per thread: ystep_e with the ADE branch, its embedded CPML,
-// the ordinary update and the PEC rule (yee.c:530-1247), then e_special --
-// the CPML psi_E update and corrections (boundary.c:691-884) and the TSF E
-// corrections (source.c:547-771).  E runs over the runs of k planes that hold a
-// dispersive cell with the plan's variant and over the rest with the plain
-// variant (SlabLists).  Each half step reads one field set and
-// writes the other, so blocks never race on a shared cell.  The *_batch
-// forms take a per-box plan index and serve many plans in one launch.
+// fdtd_kernels.cu -- the small sm_100a kernels of one GSvit FDTD time step: the
+// 1D TSF grid (aux_step, 1 CTA), the TSF face corrections, the NFFF running DFT
+// and the far-field integration.  The field updates are in fdtd_bulk.cu (TMA
+// tiles) and fdtd_flat.cu.  The *_batch forms take device tables of per-plan
+// parameters and serve many plans in one launch.
 #include <cuda_runtime.h>
 
 #include "../../include/gsvit_b200.h"
 #include "fdtd_device.cuh"
 #include "fdtd_kernels.cuh"
 
-#include "fdtd_cells.cuh"
-
 namespace {
-
-// ------------------------------------------------------------ slab kernels
-
-// One thread per cell of the slab boxes (the CPML slabs and every cell the
-// bulk kernel does not own).  slab_h forms H^{n+1/2} with the full special
-// path; slab_e then forms E^{n+1} from the H^{n+1/2} that slab_h and the bulk
-// kernel wrote.  Both read E^n/H^n from the input set only.
-
-// The box of this block: the last one whose first_block is not above
-// blockIdx.x (boxes are numbered in ascending first_block; an empty box shares
-// its successor's first_block and is skipped).  Binary search: a batch lists
-// every instance's boxes, a hundred or more.
-__device__ __forceinline__ int box_of_block(const SlabBox *boxes, int nboxes)
-{
-    const long long bid = blockIdx.x;
-    int lo = 0, hi = nboxes - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (boxes[mid].first_block <= bid) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-__device__ __forceinline__ bool box_cell(const SlabBox *boxes, int nboxes, int &i, int &j, int &k, int &inst, bool &tsf)
-{
-    const SlabBox B = boxes[box_of_block(boxes, nboxes)];
-    long long t = ((long long)blockIdx.x - B.first_block) * blockDim.x + threadIdx.x;
-    const int nk = B.k1 - B.k0, nj = B.j1 - B.j0;
-    if (t >= (long long)(B.i1 - B.i0) * nj * nk) return false;
-    k = B.k0 + (int)(t % nk);
-    t /= nk;
-    j = B.j0 + (int)(t % nj);
-    i = B.i0 + (int)(t / nj);
-    inst = B.inst;
-    tsf = B.tsf != 0;
-    return true;
-}
-
-// 3 CTAs per SM: the slab kernels are latency-bound, and 24 resident warps
-// beat the register spill this costs e_special (1.95 -> 1.60 ms per 512^3 step)
-template <class T>
-__device__ __forceinline__ void slab_h_cell(const DevPlan &P, int i, int j, int k, bool tsf)
-{
-    using R = real_t<T>;
-    const uint32_t stp = sr_step<T>(P);
-    const int64_t c = (int64_t)i * P.si + (int64_t)j * P.sj + k;
-    const float *EX = P.fin[0], *EY = P.fin[1], *EZ = P.fin[2];
-    const R ex = ldgE<T>(EX, c), ey = ldgE<T>(EY, c), ez = ldgE<T>(EZ, c);
-    const bool il = (i == P.xr - 1), jl = (j == P.yr - 1), kl = (k == P.zr - 1);
-    const R eyk = kl ? R(0) : ldgE<T>(EY, c + 1), exk = kl ? R(0) : ldgE<T>(EX, c + 1);
-    const R ezj = jl ? R(0) : ldgE<T>(EZ, c + P.sj), exj = jl ? R(0) : ldgE<T>(EX, c + P.sj);
-    const R ezi = il ? R(0) : ldgE<T>(EZ, c + P.si), eyi = il ? R(0) : ldgE<T>(EY, c + P.si);
-    R h[3] = {ldgH<T>(P, P.fin[3], c), ldgH<T>(P, P.fin[4], c), ldgH<T>(P, P.fin[5], c)};
-    const float4 *cl = reinterpret_cast<const float4 *>(P.classes);
-    h_update<T>(P, cl, cls_at(P, i, j, k), i, j, k, true, true, tsf, eyi - ey, ezi - ez, exj - ex, ezj - ez, exk - ex, eyk - ey, h);
-    stH<T>(P, P.fout[3], c, h[0], stp, 3);
-    stH<T>(P, P.fout[4], c, h[1], stp, 4);
-    stH<T>(P, P.fout[5], c, h[2], stp, 5);
-}
-
-// Four consecutive k cells per thread (boxes whose k bounds and row length
-// are multiples of 4, as all of them are next to the bulk kernel): 16-byte
-// loads of E and H, the same per-cell update as slab_h_cell with the four
-// cells' loads in flight together, 16-byte stores.
-__device__ __forceinline__ bool box_group4(const SlabBox *boxes, int nboxes, int &i, int &j, int &k, int &inst, bool &tsf)
-{
-    const SlabBox B = boxes[box_of_block(boxes, nboxes)];
-    long long t = ((long long)blockIdx.x - B.first_block) * blockDim.x + threadIdx.x;
-    const int nk = (B.k1 - B.k0) / 4, nj = B.j1 - B.j0;
-    if (t >= (long long)(B.i1 - B.i0) * nj * nk) return false;
-    k = B.k0 + 4 * (int)(t % nk);
-    t /= nk;
-    j = B.j0 + (int)(t % nj);
-    i = B.i0 + (int)(t / nj);
-    inst = B.inst;
-    tsf = B.tsf != 0;
-    return true;
-}
-
-template <class T>
-__device__ __forceinline__ void slab_h_cell4(const DevPlan &P, int i, int j, int k, bool tsf)
-{
-    const uint32_t stp = sr_step<T>(P);
-    const int64_t c = (int64_t)i * P.si + (int64_t)j * P.sj + k;
-    const float *EX = P.fin[0], *EY = P.fin[1], *EZ = P.fin[2];
-    const bool il = (i == P.xr - 1), jl = (j == P.yr - 1), kl = (k + 3 == P.zr - 1);
-    float ex[4], ey[4], ez[4], exj[4], ezj[4], eyi[4], ezi[4], hx[4], hy[4], hz[4];
-    lds4a_f(ex, ldg4_ro<T>(EX, c));
-    lds4a_f(ey, ldg4_ro<T>(EY, c));
-    lds4a_f(ez, ldg4_ro<T>(EZ, c));
-    if (jl) {
-        for (int q = 0; q < 4; q++) exj[q] = ezj[q] = 0.f;
-    } else {
-        lds4a_f(exj, ldg4_ro<T>(EX, c + P.sj));
-        lds4a_f(ezj, ldg4_ro<T>(EZ, c + P.sj));
-    }
-    if (il) {
-        for (int q = 0; q < 4; q++) eyi[q] = ezi[q] = 0.f;
-    } else {
-        lds4a_f(eyi, ldg4_ro<T>(EY, c + P.si));
-        lds4a_f(ezi, ldg4_ro<T>(EZ, c + P.si));
-    }
-    const float exk4 = kl ? 0.f : ldgE<T>(EX, c + 4), eyk4 = kl ? 0.f : ldgE<T>(EY, c + 4);
-    lds4a_f(hx, ldg4_ro<T>(P.fin[3], c));
-    lds4a_f(hy, ldg4_ro<T>(P.fin[4], c));
-    lds4a_f(hz, ldg4_ro<T>(P.fin[5], c));
-    const uint32_t cw = __ldg(reinterpret_cast<const uint32_t *>(P.cls + ((int64_t)i * P.yr + j) * P.cpitch + k));
-    const float4 *cl = reinterpret_cast<const float4 *>(P.classes);
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        float h[3] = {hx[q], hy[q], hz[q]};
-        if (Stor<T>::scaled) { h[0] *= P.ihs; h[1] *= P.ihs; h[2] *= P.ihs; }
-        const float eyk = q < 3 ? ey[q + 1] : eyk4, exk = q < 3 ? ex[q + 1] : exk4;
-        h_update<T>(P, cl, (cw >> (8 * q)) & 0xff, i, j, k + q, true, true, tsf, eyi[q] - ey[q], ezi[q] - ez[q],
-                    exj[q] - ex[q], ezj[q] - ez[q], exk - ex[q], eyk - ey[q], h);
-        hx[q] = h[0]; hy[q] = h[1]; hz[q] = h[2];
-    }
-    const float s = Stor<T>::scaled ? P.hs : 1.f;
-    stg4<T>(P.fout[3], c, make_float4(hx[0], hx[1], hx[2], hx[3]), s, stp, 3);
-    stg4<T>(P.fout[4], c, make_float4(hy[0], hy[1], hy[2], hy[3]), s, stp, 4);
-    stg4<T>(P.fout[5], c, make_float4(hz[0], hz[1], hz[2], hz[3]), s, stp, 5);
-}
-
-template <class T>
-__global__ void __launch_bounds__(256, 2) slab_h4_kernel(const __grid_constant__ DevPlan P, const SlabBox *boxes, int nboxes)
-{
-    int i, j, k, inst;
-    bool tsf;
-    if (box_group4(boxes, nboxes, i, j, k, inst, tsf)) slab_h_cell4<T>(P, i, j, k, tsf);
-}
-
-template <class T>
-__global__ void __launch_bounds__(256, 2) slab_h4_batch(const DevPlan *plans, const SlabBox *boxes, int nboxes)
-{
-    int i, j, k, inst;
-    bool tsf;
-    if (box_group4(boxes, nboxes, i, j, k, inst, tsf)) slab_h_cell4<T>(plans[inst], i, j, k, tsf);
-}
-
-template <class T>
-__global__ void __launch_bounds__(256, 3) slab_h_kernel(const __grid_constant__ DevPlan P, const SlabBox *boxes, int nboxes)
-{
-    int i, j, k, inst;
-    bool tsf;
-    if (box_cell(boxes, nboxes, i, j, k, inst, tsf)) slab_h_cell<T>(P, i, j, k, tsf);
-}
-
-template <class T>
-__global__ void __launch_bounds__(256, 3) slab_h_batch(const DevPlan *plans, const SlabBox *boxes, int nboxes)
-{
-    int i, j, k, inst;
-    bool tsf;
-    if (box_cell(boxes, nboxes, i, j, k, inst, tsf)) slab_h_cell<T>(plans[inst], i, j, k, tsf);
-}
-
-template <bool ADE, int NPOLES, class T>
-__device__ __forceinline__ void slab_e_cell(const DevPlan &P, int i, int j, int k, bool tsf)
-{
-    using R = real_t<T>;
-    const uint32_t stp = sr_step<T>(P);
-    const int64_t c = (int64_t)i * P.si + (int64_t)j * P.sj + k;
-    const float *HX = P.fout[3], *HY = P.fout[4], *HZ = P.fout[5];   // H^{n+1/2}, written this step
-    const V3<R> eo{ldgE<T>(P.fin[0], c), ldgE<T>(P.fin[1], c), ldgE<T>(P.fin[2], c)};
-    const V3<R> h{ldH<T>(P, HX, c), ldH<T>(P, HY, c), ldH<T>(P, HZ, c)};
-    const R hx_jm = j > 0 ? ldH<T>(P, HX, c - P.sj) : R(0), hz_jm = j > 0 ? ldH<T>(P, HZ, c - P.sj) : R(0);
-    const R hx_km = k > 0 ? ldH<T>(P, HX, c - 1) : R(0), hy_km = k > 0 ? ldH<T>(P, HY, c - 1) : R(0);
-    const R hy_im = i > 0 ? ldH<T>(P, HY, c - P.si) : R(0), hz_im = i > 0 ? ldH<T>(P, HZ, c - P.si) : R(0);
-    const float4 *cl = reinterpret_cast<const float4 *>(P.classes);
-    const V3<R> en =
-        e_special<ADE, NPOLES, T>(P, cl, cls_at(P, i, j, k), i, j, k, tsf, eo, h, hx_jm, hz_jm, hx_km, hy_km, hy_im, hz_im);
-    stE<T>(P.fout[0], c, en.x, stp, 0);
-    stE<T>(P.fout[1], c, en.y, stp, 1);
-    stE<T>(P.fout[2], c, en.z, stp, 2);
-}
-
-template <bool ADE, int NPOLES, class T>
-__global__ void __launch_bounds__(256, 3) slab_e_kernel(const __grid_constant__ DevPlan P, const SlabBox *boxes, int nboxes)
-{
-    int i, j, k, inst;
-    bool tsf;
-    if (box_cell(boxes, nboxes, i, j, k, inst, tsf)) slab_e_cell<ADE, NPOLES, T>(P, i, j, k, tsf);
-}
-
-template <bool ADE, int NPOLES, class T>
-__global__ void __launch_bounds__(256, 3) slab_e_batch(const DevPlan *plans, const SlabBox *boxes, int nboxes)
-{
-    int i, j, k, inst;
-    bool tsf;
-    if (box_cell(boxes, nboxes, i, j, k, inst, tsf)) slab_e_cell<ADE, NPOLES, T>(plans[inst], i, j, k, tsf);
-}
 
 // ------------------------------------------------------------ TSF face tables
 
@@ -727,42 +519,6 @@ void launch_tsf_faces(const DevPlan &p, int total, cudaStream_t st)
     if (total > 0) tsf_face_kernel<<<(total + 255) / 256, 256, 0, st>>>(p, total);
 }
 
-template <class T>
-cudaError_t slab_steps_t(const DevPlan &p, const SlabLists &L, bool ade, int npoles, cudaStream_t st, int part)
-{
-    bool h4 = false;
-    if (part & 1) {
-        if constexpr (sizeof(T) <= 4) {   // 4-cell groups: FP32 and 16-bit storage
-            if (L.h4blocks > 0) {
-                slab_h4_kernel<T><<<(unsigned)L.h4blocks, 256, 0, st>>>(p, L.h4, L.nh);
-                h4 = true;
-            }
-        }
-        if (!h4) slab_h_kernel<T><<<(unsigned)L.hblocks, 256, 0, st>>>(p, L.h, L.nh);
-    }
-    if (!(part & 2)) return cudaGetLastError();
-    if (L.eblocks > 0) {
-        if (!ade)
-            slab_e_kernel<false, 0, T><<<(unsigned)L.eblocks, 256, 0, st>>>(p, L.e, L.ne);
-        else if (npoles == 0)
-            slab_e_kernel<true, 0, T><<<(unsigned)L.eblocks, 256, 0, st>>>(p, L.e, L.ne);
-        else
-            slab_e_kernel<true, 2, T><<<(unsigned)L.eblocks, 256, 0, st>>>(p, L.e, L.ne);
-    }
-    if (L.epblocks > 0) slab_e_kernel<false, 0, T><<<(unsigned)L.epblocks, 256, 0, st>>>(p, L.ep, L.nep);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_slab_steps(const DevPlan &p, const SlabLists &L, bool ade, int npoles, int storage, cudaStream_t st,
-                              int part)
-{
-    if (L.hblocks <= 0) return cudaSuccess;
-    if (storage == FDTD_STORE_F64) return slab_steps_t<double>(p, L, ade, npoles, st, part);
-    if (storage == FDTD_STORE_F16) return slab_steps_t<__half>(p, L, ade, npoles, st, part);
-    if (storage == FDTD_STORE_BF16) return slab_steps_t<__nv_bfloat16>(p, L, ade, npoles, st, part);
-    return slab_steps_t<float>(p, L, ade, npoles, st, part);
-}
-
 void launch_aux_step_batch(const DevAux *a, int nplans, cudaStream_t st)
 {
     if (nplans > 0) aux_step_batch<<<nplans, 1024, 0, st>>>(a);
@@ -771,56 +527,6 @@ void launch_aux_step_batch(const DevAux *a, int nplans, cudaStream_t st)
 void launch_tsf_faces_batch(const DevPlan *p, int nplans, int max_cells, cudaStream_t st)
 {
     if (nplans > 0 && max_cells > 0) tsf_face_batch<<<dim3((max_cells + 255) / 256, nplans), 256, 0, st>>>(p);
-}
-
-template <class T>
-cudaError_t slab_steps_batch_t(const DevPlan *p, const SlabBox *boxes, int nboxes, long long nblocks, const SlabBox *boxes4,
-                               long long nblocks4, const SlabBox *eboxes, int neboxes, long long neblocks, bool ade,
-                               int npoles, cudaStream_t st, int part)
-{
-    if (part & 1) {
-        if (nblocks4 > 0)
-            slab_h4_batch<T><<<(unsigned)nblocks4, 256, 0, st>>>(p, boxes4, nboxes);
-        else
-            slab_h_batch<T><<<(unsigned)nblocks, 256, 0, st>>>(p, boxes, nboxes);
-    }
-    if ((part & 2) && neblocks > 0) {
-        if (!ade)
-            slab_e_batch<false, 0, T><<<(unsigned)neblocks, 256, 0, st>>>(p, eboxes, neboxes);
-        else if (npoles == 0)
-            slab_e_batch<true, 0, T><<<(unsigned)neblocks, 256, 0, st>>>(p, eboxes, neboxes);
-        else
-            slab_e_batch<true, 2, T><<<(unsigned)neblocks, 256, 0, st>>>(p, eboxes, neboxes);
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_slab_steps_batch(const DevPlan *p, const SlabBox *boxes, int nboxes, long long nblocks,
-                                    const SlabBox *boxes4, long long nblocks4, const SlabBox *eboxes, int neboxes,
-                                    long long neblocks, bool ade, int npoles, int storage, cudaStream_t st, int part)
-{
-    if (nblocks <= 0) return cudaSuccess;
-    if (storage == FDTD_STORE_F16)
-        return slab_steps_batch_t<__half>(p, boxes, nboxes, nblocks, boxes4, nblocks4, eboxes, neboxes, neblocks, ade, npoles, st,
-                                          part);
-    if (storage == FDTD_STORE_BF16)
-        return slab_steps_batch_t<__nv_bfloat16>(p, boxes, nboxes, nblocks, boxes4, nblocks4, eboxes, neboxes, neblocks, ade,
-                                                 npoles, st, part);
-    return slab_steps_batch_t<float>(p, boxes, nboxes, nblocks, boxes4, nblocks4, eboxes, neboxes, neblocks, ade, npoles, st,
-                                     part);
-}
-
-cudaError_t launch_slab_e_plain_batch(const DevPlan *p, const SlabBox *boxes, int nboxes, long long nblocks, int storage,
-                                      cudaStream_t st)
-{
-    if (nblocks <= 0) return cudaSuccess;
-    if (storage == FDTD_STORE_F16)
-        slab_e_batch<false, 0, __half><<<(unsigned)nblocks, 256, 0, st>>>(p, boxes, nboxes);
-    else if (storage == FDTD_STORE_BF16)
-        slab_e_batch<false, 0, __nv_bfloat16><<<(unsigned)nblocks, 256, 0, st>>>(p, boxes, nboxes);
-    else
-        slab_e_batch<false, 0, float><<<(unsigned)nblocks, 256, 0, st>>>(p, boxes, nboxes);
-    return cudaGetLastError();
 }
 
 void launch_nfff_accumulate_batch(const DevNfff *n, int nplans, int max_cells, cudaStream_t st)

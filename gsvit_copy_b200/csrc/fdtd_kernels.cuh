@@ -44,55 +44,15 @@ struct DevNfff {
     int storage;                // FDTD_STORE_* of the fields
 };
 
-// a box of cells; its blocks are [first_block, next box's first_block), one cell
-// (or one 4-cell group in a 4-cell list) per thread
-struct SlabBox {
-    int i0, i1, j0, j1, k0, k1;
-    long long first_block;
-    int inst;                   // plan of the box in a batched launch
-    int tsf;                    // 1 if the box meets the TSF correction region [t0 - 1, t1] on every axis;
-                                // the cells of other boxes skip the TSF test
-};
-
 void launch_aux_step(const DevAux &a, cudaStream_t st);
 
 // Batched forms: one launch covers many plans whose per-plan parameters are
 // device tables (of this step's parity), indexed by the plan number.
 void launch_aux_step_batch(const DevAux *a, int nplans, cudaStream_t st);
 void launch_tsf_faces_batch(const DevPlan *p, int nplans, int max_cells, cudaStream_t st);
-// H over boxes (or boxes4 in 4-cell groups, nblocks4 > 0) and E over eboxes,
-// the instances' runs of k planes with a dispersive cell (SlabLists::e)
-// part: 1 the H kernel, 2 the E kernel over the dispersive runs, 3 both
-cudaError_t launch_slab_steps_batch(const DevPlan *p, const SlabBox *boxes, int nboxes, long long nblocks,
-                                    const SlabBox *boxes4, long long nblocks4, const SlabBox *eboxes, int neboxes,
-                                    long long neblocks, bool ade, int npoles, int storage, cudaStream_t st, int part = 3);
-// E over every instance's runs without a dispersive cell (SlabLists::ep)
-cudaError_t launch_slab_e_plain_batch(const DevPlan *p, const SlabBox *boxes, int nboxes, long long nblocks, int storage,
-                                      cudaStream_t st);
 void launch_nfff_accumulate_batch(const DevNfff *n, int nplans, int max_cells, cudaStream_t st);
 void launch_probe_capture(const DevAux &a, cudaStream_t st);
 void launch_tsf_faces(const DevPlan &p, int total, cudaStream_t st);
-// The slab work lists of a plan.  H runs over every slab box, in 4-cell
-// groups when h4blocks > 0 (every k bound and the row length multiples of 4).
-// E runs over the same cells split along k: `e` holds the runs of k planes
-// with a dispersive cell (the plan's E variant), `ep` the runs without one
-// (the plain E variant, fewer registers); without a split `e` is every box.
-struct SlabLists {
-    const SlabBox *h;
-    int nh;
-    long long hblocks;
-    const SlabBox *h4;
-    long long h4blocks;
-    const SlabBox *e;
-    int ne;
-    long long eblocks;
-    const SlabBox *ep;
-    int nep;
-    long long epblocks;
-};
-// part: 1 the H kernel, 2 the E kernels, 3 both (in that order)
-cudaError_t launch_slab_steps(const DevPlan &p, const SlabLists &L, bool ade, int npoles, int storage, cudaStream_t st,
-                              int part = 3);
 void launch_nfff_accumulate(const DevNfff &n, cudaStream_t st);
 // folds the samples of the steps since the last multiple of NFFF_RING into the
 // accumulators and clears their ring slots; due before the accumulators are read
