@@ -508,7 +508,66 @@ __global__ void nfff_series_kernel(const DevNfffSeries S)
     }
 }
 
+// ------------------------------------------------------------ host copies
+
+// Host values to and from the storage type: double to float first (FP64 storage
+// keeps the double), then to nearest; H components carry the 16-bit scale.  PCIe
+// bounds the copies around these by 100 times.
+template <class T, class H>
+__global__ void pack_kernel(const H *src, T *dst, size_t n, float scale)
+{
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
+        if constexpr (sizeof(T) == 8) dst[q] = (T)src[q];
+        else Stor<T>::st(reinterpret_cast<float *>(dst), (int64_t)q, (float)src[q] * scale);
+    }
+}
+
+template <class T, class H>
+__global__ void unpack_kernel(const T *src, H *dst, size_t n, float scale)
+{
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
+        if constexpr (sizeof(T) == 8) dst[q] = (H)src[q];
+        else dst[q] = (H)(Stor<T>::ld(reinterpret_cast<const float *>(src), (int64_t)q) * scale);
+    }
+}
+
+unsigned copy_grid(size_t n) { return (unsigned)((n + 1023) / 1024 < 148 * 8 ? (n + 1023) / 1024 : 148 * 8); }
+
+template <class T>
+void pack_t(int hsz, const void *host, float *field, size_t off, size_t n, float scale, cudaStream_t st)
+{
+    T *f = reinterpret_cast<T *>(field) + off;
+    if (hsz == 4) pack_kernel<<<copy_grid(n), 256, 0, st>>>(static_cast<const float *>(host), f, n, scale);
+    else pack_kernel<<<copy_grid(n), 256, 0, st>>>(static_cast<const double *>(host), f, n, scale);
+}
+
+template <class T>
+void unpack_t(int hsz, const float *field, size_t off, void *host, size_t n, float scale, cudaStream_t st)
+{
+    const T *f = reinterpret_cast<const T *>(field) + off;
+    if (hsz == 4) unpack_kernel<<<copy_grid(n), 256, 0, st>>>(f, static_cast<float *>(host), n, scale);
+    else unpack_kernel<<<copy_grid(n), 256, 0, st>>>(f, static_cast<double *>(host), n, scale);
+}
+
 }  // namespace
+
+void launch_pack(int storage, int hsz, const void *host, float *field, size_t off, size_t n, float scale, cudaStream_t st)
+{
+    if (n == 0) return;
+    if (storage == FDTD_STORE_F64) pack_t<double>(hsz, host, field, off, n, scale, st);
+    else if (storage == FDTD_STORE_F16) pack_t<__half>(hsz, host, field, off, n, scale, st);
+    else if (storage == FDTD_STORE_BF16) pack_t<__nv_bfloat16>(hsz, host, field, off, n, scale, st);
+    else pack_t<float>(hsz, host, field, off, n, scale, st);
+}
+
+void launch_unpack(int storage, int hsz, const float *field, size_t off, void *host, size_t n, float scale, cudaStream_t st)
+{
+    if (n == 0) return;
+    if (storage == FDTD_STORE_F64) unpack_t<double>(hsz, field, off, host, n, scale, st);
+    else if (storage == FDTD_STORE_F16) unpack_t<__half>(hsz, field, off, host, n, scale, st);
+    else if (storage == FDTD_STORE_BF16) unpack_t<__nv_bfloat16>(hsz, field, off, host, n, scale, st);
+    else unpack_t<float>(hsz, field, off, host, n, scale, st);
+}
 
 void launch_aux_step(const DevAux &a, cudaStream_t st) { aux_step_kernel<<<1, 1024, 0, st>>>(a); }
 

@@ -52,6 +52,11 @@ void launch_aux_step_batch(const DevAux *a, int nplans, cudaStream_t st);
 void launch_tsf_faces_batch(const DevPlan *p, int nplans, int max_cells, cudaStream_t st);
 void launch_nfff_accumulate_batch(const DevNfff *n, int nplans, int max_cells, cudaStream_t st);
 void launch_probe_capture(const DevAux &a, cudaStream_t st);
+// n host values (hsz bytes each: 4 float, 8 double) at `host`, device memory, to
+// and from elements off .. off+n-1 of a field stored as FDTD_STORE_*; the field
+// holds `scale` times the value (pack), or `scale` undoes that (unpack)
+void launch_pack(int storage, int hsz, const void *host, float *field, size_t off, size_t n, float scale, cudaStream_t st);
+void launch_unpack(int storage, int hsz, const float *field, size_t off, void *host, size_t n, float scale, cudaStream_t st);
 void launch_tsf_faces(const DevPlan &p, int total, cudaStream_t st);
 void launch_nfff_accumulate(const DevNfff &n, cudaStream_t st);
 // folds the samples of the steps since the last multiple of NFFF_RING into the

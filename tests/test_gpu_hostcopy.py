@@ -1,0 +1,46 @@
+"""Host copies that change the element type (fdtd_set_fields / fdtd_get_fields
+and their FP32 forms) convert on the device, in chunks of the staging buffer
+(2^22 doubles, 2^23 floats).  Against numpy / torch conversions, bit for bit, on
+a grid of more than one chunk and on one smaller than a block: double to float,
+then to the storage type to nearest (H times 2^9 at 16 bits); FP64 storage keeps
+doubles."""
+import numpy as np
+import pytest
+import torch
+
+from gsvit_copy_b200 import abi, plan
+from gsvit_copy_b200.solver import Solver
+from tests._util import random_fields
+
+pytestmark = pytest.mark.gpu
+
+
+def _stored(x, storage, scale):
+    if storage == abi.STORE_F64:
+        return x
+    f = x.astype(np.float32)
+    if storage == abi.STORE_F32:
+        return f.astype(np.float64)
+    t = torch.float16 if storage == abi.STORE_F16 else torch.bfloat16
+    v = torch.from_numpy(f * np.float32(scale)).to(t).to(torch.float32).numpy() / np.float32(scale)
+    return v.astype(np.float64)
+
+
+@pytest.mark.parametrize("storage", [abi.STORE_F32, abi.STORE_F16, abi.STORE_BF16, abi.STORE_F64],
+                         ids=["f32", "f16", "bf16", "f64"])
+@pytest.mark.parametrize("shape", [(9, 7, 5), (172, 170, 291)])   # 315 and 8.5 M cells
+def test_round_trip_bits(shape, storage):
+    dx = 10e-9
+    s = plan.Scene(name="copy", xres=shape[0], yres=shape[1], zres=shape[2], dx=dx, dt=plan.plan_dt(dx, dx, dx, 0.5), nsteps=1)
+    s.mats = [plan.vacuum_material()]
+    s.mat = np.zeros(shape, dtype=np.int32)
+    s.storage = storage
+    g = Solver(s)
+    init = random_fields(shape, 8)
+    g.set_fields(init)
+    want = [_stored(np.asarray(c, dtype=np.float64), storage, 1.0 if q < 3 else 512.0) for q, c in enumerate(init)]
+    for a, b in zip(g.fields(), want):
+        assert np.array_equal(a, b)
+    for a, b in zip(g.fields(dtype=np.float32), want):
+        assert np.array_equal(a, b.astype(np.float32))
+    g.close()
