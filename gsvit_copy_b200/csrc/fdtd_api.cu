@@ -73,6 +73,10 @@ struct DevBuf {        // a list of device allocations freed with the plan
     }
 };
 
+struct TsfTab {        // the TSF corrections of one step
+    float2 *h[6], *e[6];
+};
+
 struct SnapItem {      // one contiguous device range that is part of the stepping state
     void *ptr;
     size_t bytes;
@@ -120,6 +124,11 @@ struct fdtd_plan {
     double tile_bytes[NTILE] = {};         // algorithmic HBM bytes per launch of each tile kind
     char *stage = nullptr;                // staging of the host copies that change the element type
     size_t stage_bytes = 0;
+    // what a step needs and leaves (1D grid and TSF tables; NFFF) beside the steps
+    // around it (run_steps)
+    cudaStream_t prep = nullptr, post = nullptr;
+    cudaEvent_t ev_main = nullptr, ev_prep = nullptr, ev_post = nullptr;
+    TsfTab tab[2] = {};                   // TSF correction tables of even and odd steps of a call
     int *d_err = nullptr;                 // set by a bulk CTA whose bounded wait expired
     const int *batch_err = nullptr;       // the batch's error word, for an instance of a batch
     bool failed = false;                  // an expired wait was reported: the plan only accepts destroy
@@ -198,9 +207,8 @@ int launch_tile_kind(fdtd_plan *P, const DevPlan &d, int in, int kind, cudaStrea
 // the Yee/CPML/TSF/ADE part of one step: the TMA tiles (bulk, then the CPML
 // tiles; they touch disjoint cells and read only the input set), or, for
 // plans without them, the bulk box and the flat kernels, or the flat kernels alone
-int launch_fused(fdtd_plan *P, int in, cudaStream_t st)
+int launch_fused(fdtd_plan *P, const DevPlan &d, int in, cudaStream_t st)
 {
-    DevPlan d = plan_for(P, in);
     cudaError_t e;
     if (P->tiles_on) {
         // the four kinds touch disjoint cells and read only the input set:
@@ -251,35 +259,111 @@ int launch_fused(fdtd_plan *P, int in, cudaStream_t st)
     return FDTD_OK;
 }
 
-// NFFF work of a step: running DFT and/or the exact time-domain series,
-// both reading the E set this step wrote
-void launch_nfff(fdtd_plan *P, int in, cudaStream_t st)
+// ---- the parts of step `off` of a call.  The device step counter holds the
+// steps done before the call until close_steps advances it, so that no part of
+// a step waits for another only to learn its number.
+
+// the plan as step `off` sees it: input set `in`, TSF tables `tab`
+DevPlan plan_at(const fdtd_plan *P, int in, int off, const TsfTab &tab)
+{
+    DevPlan d = plan_for(P, in);
+    d.step_off = off + 1;
+    for (int f = 0; f < 6; f++) {
+        d.tcor_h[f] = tab.h[f];
+        d.tcor_e[f] = tab.e[f];
+    }
+    return d;
+}
+
+// 1D TSF grid and face corrections of step `off`; the probes of step off - 2,
+// whose fields are in set `last`
+void launch_prep(fdtd_plan *P, int off, int last, const TsfTab &tab, cudaStream_t st)
+{
+    if (!P->aux.res && !P->aux.nprobes) return;
+    DevAux a = P->aux;
+    a.off = off;
+    a.fields = P->d_fieldptrs[last];
+    launch_aux_line(a, st);
+    if (P->tsf_cells) launch_tsf_faces(plan_at(P, 0, off, tab), P->tsf_cells, st);
+}
+
+// NFFF work of step `off`, which wrote set `out`: running DFT and/or the exact
+// time-domain series
+void launch_nfff(fdtd_plan *P, int off, int out, cudaStream_t st)
 {
     if (!P->nfff) return;
     if (P->nfff_nfreq > 0) {
         DevNfff n = P->nf;
-        n.e = P->d_efieldptrs[1 - in];
+        n.off = off;
+        n.e = P->d_efieldptrs[out];
         launch_nfff_accumulate(n, st);
     }
     if (P->nfff_series) {
         DevNfffSeries q = P->ns;
-        q.e = P->d_efieldptrs[1 - in];
+        q.off = off;
+        q.e = P->d_efieldptrs[out];
         launch_nfff_series(q, st);
     }
 }
 
-int launch_step(fdtd_plan *P, cudaStream_t st)
+// the end of a call of n steps: the probes of its last two, the step counter
+void close_steps(fdtd_plan *P, int n, cudaStream_t st)
 {
-    const int in = P->cur;
     DevAux a = P->aux;
-    a.fields = P->d_fieldptrs[in];
-    launch_aux_step(a, st);
-    if (P->tsf_cells) launch_tsf_faces(P->dp, P->tsf_cells, st);
-    int rc = launch_fused(P, in, st);
-    if (rc != FDTD_OK) return rc;
-    launch_nfff(P, in, st);
-    P->cur = 1 - in;
+    a.off = n;
+    a.fields = P->d_fieldptrs[P->cur];
+    launch_close_steps(a, P->d_fieldptrs[1 - P->cur], st);
+}
+
+// n steps on `st`.  Only the field updates of a step follow from the last
+// step's: its 1D grid and TSF tables are made during the step before it, and
+// the NFFF work of a step runs during the next, on two side streams (64^3 rough
+// surface: 30 -> 20 us a step, 256^3: 393 -> 381, 512^3: 2310 -> 2270).  Two
+// sets of TSF tables alternate.  `tab`: one set for all steps, everything in
+// order on `st` (fdtd_step_static_scratch).  `after` (if set) is called after
+// the field update of each step with its input set.
+template <class F>
+int run_steps(fdtd_plan *P, int n, cudaStream_t st, const TsfTab *tab, F after)
+{
+    if (n <= 0) return FDTD_OK;
+    const bool piped = !tab;
+    const bool has_prep = P->aux.res || P->aux.nprobes, has_post = P->nfff;
+    const int c0 = P->cur;
+    auto set_in = [&](int s) { return (c0 + s) & 1; };           // step s reads this set, writes the other
+    auto tables = [&](int s) -> const TsfTab & { return tab ? *tab : P->tab[s & 1]; };
+    launch_prep(P, 0, 0, tables(0), st);
+    for (int s = 0; s < n; s++) {
+        const bool pre = piped && has_prep && s + 1 < n, pst = piped && has_post && s > 0;
+        if (pre || pst) CK(cudaEventRecord(P->ev_main, st));
+        if (pre) {   // the tables of step s + 1 were last read by step s - 1
+            CK(cudaStreamWaitEvent(P->prep, P->ev_main, 0));
+            launch_prep(P, s + 1, set_in(s), tables(s + 1), P->prep);
+            CK(cudaEventRecord(P->ev_prep, P->prep));
+        }
+        if (pst) {   // step s - 1's fields: read by step s, written by step s + 1
+            CK(cudaStreamWaitEvent(P->post, P->ev_main, 0));
+            launch_nfff(P, s - 1, set_in(s), P->post);
+            CK(cudaEventRecord(P->ev_post, P->post));
+        }
+        if (!piped && s > 0) launch_prep(P, s, set_in(s - 1), tables(s), st);
+        const int in = set_in(s);
+        const int rc = launch_fused(P, plan_at(P, in, s, tables(s)), in, st);
+        if (rc != FDTD_OK) return rc;
+        after(in, s);
+        P->cur = 1 - in;
+        if (pre) CK(cudaStreamWaitEvent(st, P->ev_prep, 0));
+        if (pst) CK(cudaStreamWaitEvent(st, P->ev_post, 0));
+        if (!piped) launch_nfff(P, s, 1 - in, st);
+    }
+    if (piped) launch_nfff(P, n - 1, P->cur, st);
+    close_steps(P, n, st);
+    CK(cudaGetLastError());
     return FDTD_OK;
+}
+
+int run_steps(fdtd_plan *P, int n, cudaStream_t st, const TsfTab *tab = nullptr)
+{
+    return run_steps(P, n, st, tab, [](int, int) {});
 }
 
 int final_probes(fdtd_plan *P, cudaStream_t st)
@@ -647,6 +731,14 @@ std::vector<FlatBlock> flat_blocks(const HostPlan &hp, const DevPlan &d, const i
     return flat_emit(pieces);
 }
 
+void side_free(fdtd_plan *P)
+{
+    for (cudaStream_t s : {P->prep, P->post})
+        if (s) { cudaStreamSynchronize(s); cudaStreamDestroy(s); }
+    for (cudaEvent_t e : {P->ev_main, P->ev_prep, P->ev_post})
+        if (e) cudaEventDestroy(e);
+}
+
 int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool pole_arrays)
 {
     if (!out) return fail(FDTD_E_INVALID, "out is NULL");
@@ -674,6 +766,7 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
             if (P->ev_join[k]) cudaEventDestroy(P->ev_join[k]);
         }
         if (P->ev_fork) cudaEventDestroy(P->ev_fork);
+        side_free(P);
         P->mem.free_all();
         if (P->own_stream) cudaStreamDestroy(P->own_stream);
         delete P;
@@ -690,6 +783,13 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
 #define CA(x, what) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) return bail(e_, what); } while (0)
     CA(cudaStreamCreateWithFlags(&P->own_stream, cudaStreamNonBlocking), "stream");
     P->stream = P->own_stream;
+    {   // the side streams' few blocks go ahead of the field kernels' many
+        int least = 0, most = 0;
+        CA(cudaDeviceGetStreamPriorityRange(&least, &most), "stream priorities");
+        CA(cudaStreamCreateWithPriority(&P->prep, cudaStreamNonBlocking, most), "stream");
+        CA(cudaStreamCreateWithPriority(&P->post, cudaStreamNonBlocking, most), "stream");
+        for (cudaEvent_t *e : {&P->ev_main, &P->ev_prep, &P->ev_post}) CA(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "events");
+    }
     const size_t n = hp.n;
     DevPlan &d = P->dp;
     std::memset(&d, 0, sizeof(d));
@@ -838,8 +938,12 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
             uint8_t *m;
             CA(upload(P->mem, &m, hp.tmap[f].data(), hp.tmap[f].size()), "tsf map");
             d.tmap[f] = m;
-            CA(P->mem.alloc(&d.tcor_h[f], hp.tmap[f].size() * rsz / 4), "tsf corrections");   // float2 / double2
-            CA(P->mem.alloc(&d.tcor_e[f], hp.tmap[f].size() * rsz / 4), "tsf corrections");
+            for (TsfTab &tb : P->tab) {   // float2 / double2
+                CA(P->mem.alloc(&tb.h[f], hp.tmap[f].size() * rsz / 4), "tsf corrections");
+                CA(P->mem.alloc(&tb.e[f], hp.tmap[f].size() * rsz / 4), "tsf corrections");
+            }
+            d.tcor_h[f] = P->tab[0].h[f];
+            d.tcor_e[f] = P->tab[0].e[f];
             d.tnb[f] = hp.tmap_dims[f][1];
             P->tsf_cells += (int)hp.tmap[f].size();
         }
@@ -1015,6 +1119,7 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
             P->nf.acc = acc;
             P->nf.omega_dt = dodt;
             P->nf.step = P->d_step;
+            P->nf.off = -1;   // batches, whose counter is ahead by one
             P->nf.storage = P->storage;
             P->nf.inv2dx = 1.0 / (2.0 * hp.dx);
             P->ff.npoints = f.npoints;
@@ -1269,6 +1374,7 @@ int fdtd_plan_destroy(fdtd_plan *P)
         if (P->ev_join[k]) cudaEventDestroy(P->ev_join[k]);
     }
     if (P->ev_fork) cudaEventDestroy(P->ev_fork);
+    side_free(P);
     P->mem.free_all();
     if (P->own_stream) cudaStreamDestroy(P->own_stream);
     delete P;
@@ -1372,14 +1478,9 @@ int fdtd_step(fdtd_plan *P, int nsteps)
     if (!P || nsteps < 0) return fail(FDTD_E_INVALID, "bad argument");
     if (P->failed) return refuse_failed(P);
     CK(cudaSetDevice(P->device));
-    for (int s = 0; s < nsteps; s++) {
-        int rc = launch_step(P, P->stream);
-        if (rc != FDTD_OK) return rc;
-        P->host_step++;
-    }
-    final_probes(P, P->stream);
-    CK(cudaGetLastError());
-    return FDTD_OK;
+    const int rc = run_steps(P, nsteps, P->stream);
+    if (rc == FDTD_OK) P->host_step += nsteps;
+    return rc;
 }
 
 }  // extern "C"
@@ -1426,7 +1527,7 @@ int fdtd_step_static_scratch(fdtd_plan *P, int nsteps)
     int rc = static_scratch_addr(P->device, &base);
     if (rc != FDTD_OK) return rc;
     // carve the twelve tables (H and E corrections of six faces) out of the array
-    float2 *th[6] = {}, *te[6] = {};
+    TsfTab tab = {};
     size_t used = 0;
     if (P->tsf_cells) {
         for (int f = 0; f < 6; f++) {
@@ -1435,33 +1536,14 @@ int fdtd_step_static_scratch(fdtd_plan *P, int nsteps)
             if (used + 2 * bytes > FDTD_STATIC_SCRATCH_BYTES)
                 return fail(FDTD_E_UNSUPPORTED, "the TSF face tables of this plan need more than the "
                                                 "FDTD_STATIC_SCRATCH_BYTES (32 MiB) of static scratch");
-            th[f] = reinterpret_cast<float2 *>(base + used);
-            te[f] = reinterpret_cast<float2 *>(base + used + bytes);
+            tab.h[f] = reinterpret_cast<float2 *>(base + used);
+            tab.e[f] = reinterpret_cast<float2 *>(base + used + bytes);
             used += 2 * bytes;
         }
     }
-    float2 *keep_h[6], *keep_e[6];
-    for (int f = 0; f < 6; f++) {
-        keep_h[f] = P->dp.tcor_h[f];
-        keep_e[f] = P->dp.tcor_e[f];
-        if (P->tsf_cells) {
-            P->dp.tcor_h[f] = th[f];
-            P->dp.tcor_e[f] = te[f];
-        }
-    }
-    rc = FDTD_OK;
-    for (int s = 0; s < nsteps && rc == FDTD_OK; s++) {
-        rc = launch_step(P, P->stream);
-        if (rc == FDTD_OK) P->host_step++;
-    }
-    for (int f = 0; f < 6; f++) {
-        P->dp.tcor_h[f] = keep_h[f];
-        P->dp.tcor_e[f] = keep_e[f];
-    }
-    if (rc != FDTD_OK) return rc;
-    final_probes(P, P->stream);
-    CK(cudaGetLastError());
-    return FDTD_OK;
+    rc = run_steps(P, nsteps, P->stream, &tab);
+    if (rc == FDTD_OK) P->host_step += nsteps;
+    return rc;
 }
 
 int fdtd_step_graph(fdtd_plan *P, int nsteps, int chunk)
@@ -1483,12 +1565,11 @@ int fdtd_step_graph(fdtd_plan *P, int nsteps, int chunk)
             cudaGraph_t g;
             cudaStream_t cs = P->stream;
             CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-            for (int s = 0; s < chunk; s++) {
-                int rc = launch_step(P, cs);
-                if (rc != FDTD_OK) {
-                    cudaStreamEndCapture(cs, &g);
-                    return rc;
-                }
+            const int rc = run_steps(P, chunk, cs);
+            if (rc != FDTD_OK) {
+                cudaStreamEndCapture(cs, &g);
+                P->cur = par;
+                return rc;
             }
             CK(cudaStreamEndCapture(cs, &g));
             cudaGraphExec_t ge;
@@ -1502,14 +1583,9 @@ int fdtd_step_graph(fdtd_plan *P, int nsteps, int chunk)
         done += chunk;
         P->host_step += chunk;
     }
-    for (; done < nsteps; done++) {
-        int rc = launch_step(P, P->stream);
-        if (rc != FDTD_OK) return rc;
-        P->host_step++;
-    }
-    final_probes(P, P->stream);
-    CK(cudaGetLastError());
-    return FDTD_OK;
+    const int rc = run_steps(P, nsteps - done, P->stream);
+    if (rc == FDTD_OK) P->host_step += nsteps - done;
+    return rc;
 }
 
 int fdtd_get_step(const fdtd_plan *P, int *step)
@@ -1528,19 +1604,16 @@ int fdtd_step_timed(fdtd_plan *P, int nsteps, double *fused_ms, int *fused_launc
     for (auto &e : ev) CK(cudaEventCreate(&e));
     for (int s = 0; s < nsteps; s++) {
         const int in = P->cur;
-        DevAux a = P->aux;
-        a.fields = P->d_fieldptrs[in];
-        launch_aux_step(a, P->stream);
-        if (P->tsf_cells) launch_tsf_faces(P->dp, P->tsf_cells, P->stream);
+        launch_prep(P, 0, 0, P->tab[0], P->stream);
         CK(cudaEventRecord(ev[2 * s], P->stream));
-        int rc = launch_fused(P, in, P->stream);
+        int rc = launch_fused(P, plan_at(P, in, 0, P->tab[0]), in, P->stream);
         CK(cudaEventRecord(ev[2 * s + 1], P->stream));
         if (rc != FDTD_OK) return rc;
-        launch_nfff(P, in, P->stream);
+        launch_nfff(P, 0, 1 - in, P->stream);
         P->cur = 1 - in;
+        close_steps(P, 1, P->stream);
         P->host_step++;
     }
-    final_probes(P, P->stream);
     CK(cudaStreamSynchronize(P->stream));
     double tot = 0;
     for (int s = 0; s < nsteps; s++) {
@@ -1566,13 +1639,10 @@ int fdtd_step_profile(fdtd_plan *P, int nsteps, double out[8])
     for (int s = 0; s < nsteps; s++) {
         cudaEvent_t *E = &ev[(size_t)NE * s];
         const int in = P->cur;
-        DevAux a = P->aux;
-        a.fields = P->d_fieldptrs[in];
         CK(cudaEventRecord(E[0], st));
-        launch_aux_step(a, st);
-        if (P->tsf_cells) launch_tsf_faces(P->dp, P->tsf_cells, st);
+        launch_prep(P, 0, 0, P->tab[0], st);
         CK(cudaEventRecord(E[1], st));
-        DevPlan d = plan_for(P, in);
+        const DevPlan d = plan_at(P, in, 0, P->tab[0]);
         if (P->tiles_on) {
             int rc = launch_tile_kind(P, d, in, TILE_BULK, st);
             if (rc != FDTD_OK) return rc;
@@ -1593,12 +1663,12 @@ int fdtd_step_profile(fdtd_plan *P, int nsteps, double out[8])
             if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("flat step launch: ") + cudaGetErrorString(e));
         }
         CK(cudaEventRecord(E[3], st));
-        launch_nfff(P, in, st);
+        launch_nfff(P, 0, 1 - in, st);
         CK(cudaEventRecord(E[4], st));
         P->cur = 1 - in;
+        close_steps(P, 1, st);
         P->host_step++;
     }
-    final_probes(P, st);
     CK(cudaStreamSynchronize(st));
     double aux = 0, bulk = 0, slab = 0, nf = 0, tot = 0;
     for (int s = 0; s < nsteps; s++) {
@@ -2402,13 +2472,13 @@ int fdtd_adjoint_gradient(fdtd_plan *P, const fdtd_objective *obj, int nsteps, i
         if (e != cudaSuccess) return fail(FDTD_E_NOMEM, std::string("adjoint checkpoints: ") + cudaGetErrorString(e));
     }
     // forward pass with a checkpoint at the start of every segment
-    for (int m = 0; m < nsteps; m++) {
-        if (m % K == 0) CK(ckpt_save(P, ck, m / K));
-        rc = launch_step(P, P->stream);
+    for (int seg = 0; seg < nseg; seg++) {
+        const int len = std::min(K, nsteps - seg * K);
+        CK(ckpt_save(P, ck, seg));
+        rc = run_steps(P, len, P->stream);
         if (rc != FDTD_OK) return rc;
-        P->host_step++;
+        P->host_step += len;
     }
-    final_probes(P, P->stream);
     CK(ckpt_save(P, ck, nseg));
     launch_nfff_fold_pending(P->nf, P->stream);
     launch_farfield_finalize(P->ff, P->stream);
@@ -2449,12 +2519,10 @@ int fdtd_adjoint_gradient(fdtd_plan *P, const fdtd_objective *obj, int nsteps, i
     for (int seg = nseg - 1; seg >= 0; seg--) {
         const int m0 = seg * K, m1 = std::min(nsteps, m0 + K);
         CK(ckpt_restore(P, ck, seg));
-        for (int m = m0; m < m1; m++) {
-            rc = launch_step(P, P->stream);
-            if (rc != FDTD_OK) return rc;
-            P->host_step++;
-            launch_design_curl(plan_for(P, 1 - P->cur), g, m - m0, P->stream);
-        }
+        rc = run_steps(P, m1 - m0, P->stream, nullptr,
+                       [&](int in, int s) { launch_design_curl(plan_for(P, in), g, s, P->stream); });
+        if (rc != FDTD_OK) return rc;
+        P->host_step += m1 - m0;
         for (int m = m1 - 1; m >= m0; m--) adj_step_back(P, B, &o, m, &g, m - m0);
         CK(cudaGetLastError());
     }

@@ -179,7 +179,7 @@ struct Tab<double> {
 template <class T>
 __device__ __forceinline__ uint32_t sr_step(const DevPlan &P)
 {
-    if constexpr (Stor<T>::stochastic) return (uint32_t)__ldg(P.stepc);
+    if constexpr (Stor<T>::stochastic) return (uint32_t)(__ldg(P.stepc) + P.step_off);
     else return 0u;
 }
 template <class T>

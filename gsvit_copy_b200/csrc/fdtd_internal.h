@@ -107,7 +107,8 @@ struct DevPlan {
     // exact); FP32 storage uses none of them.  The field and psi pointers
     // below then point to 16-bit elements.
     float hs, ihs, ps, ips, pse, ipse;
-    const int *stepc;               // device step counter (seeds the BF16 stochastic rounding)
+    const int *stepc;               // device step counter; *stepc + step_off seeds the BF16 stochastic rounding
+    int step_off;
     // fields: [0..2] = E x,y,z, [3..5] = H x,y,z
     const float *fin[6];
     float *fout[6];

@@ -120,53 +120,69 @@ __global__ void tsf_face_batch(const DevPlan *plans)
 // 1D TSF grid step of source.c:1469-1473 over 1dpool.c:84-162, in FP64 with
 // the reference's operation order (no contraction); also records the probes
 // of the previous step (output.c:341-352).
-__device__ __forceinline__ void aux_step_body(const DevAux &A)
+__device__ __forceinline__ void aux_line(const DevAux &A, int s)
 {
-    const int s = *A.step;
+    if (A.res <= 0) return;
     const int tid = threadIdx.x, nt = blockDim.x;
-    if (s > 0 && s - 1 < A.nsteps_planned) {
-        for (int q = tid; q < A.nprobes * 6; q += nt) {
-            int p = q / 6, comp = q % 6;
-            A.probe_out[((size_t)p * A.nsteps_planned + (s - 1)) * 6 + comp] = ld_any(A.fields[comp], A.probe_cells[p], A.storage) * (comp >= 3 ? (double)A.ihs : 1.0);
-        }
-    }
-    if (A.res > 0) {
-        double *e = A.e, *h = A.h;
-        const int r = A.res;
-        for (int i = 1 + tid; i < r; i += nt)               // sv_1dpool_ystep_e
-            e[i] = __dadd_rn(e[i], __dmul_rn(A.ce, __dadd_rn(h[i - 1], -h[i])));
-        __syncthreads();
-        if (tid == 0) {
-            double *b = A.bnd;
-            e[0] = __dadd_rn(b[1], __dmul_rn(A.lc, __dadd_rn(e[1], -b[0])));          // sv_1dpool_boundary
-            h[0] = __dadd_rn(b[3], __dmul_rn(A.lc, __dadd_rn(h[1], -b[2])));
-            e[r - 1] = __dadd_rn(b[5], __dmul_rn(A.lc, __dadd_rn(e[r - 2], -b[4])));
-            h[r - 1] = __dadd_rn(b[7], __dmul_rn(A.lc, __dadd_rn(h[r - 2], -b[6])));
-            b[0] = e[0]; b[1] = e[1]; b[2] = h[0]; b[3] = h[1];                          // _boundary_copy
-            b[4] = e[r - 1]; b[5] = e[r - 2]; b[6] = h[r - 1]; b[7] = h[r - 2];
-            e[0] = (s < A.nwave) ? A.wave[s] : 0.0;                                        // _apply_source
-        }
-        __syncthreads();
-        for (int i = tid; i < r - 1; i += nt)               // sv_1dpool_ystep_h
-            h[i] = __dadd_rn(h[i], __dmul_rn(A.chh, __dadd_rn(e[i], -e[i + 1])));
+    double *e = A.e, *h = A.h;
+    const int r = A.res;
+    for (int i = 1 + tid; i < r; i += nt)               // sv_1dpool_ystep_e
+        e[i] = __dadd_rn(e[i], __dmul_rn(A.ce, __dadd_rn(h[i - 1], -h[i])));
+    __syncthreads();
+    if (tid == 0) {
+        double *b = A.bnd;
+        e[0] = __dadd_rn(b[1], __dmul_rn(A.lc, __dadd_rn(e[1], -b[0])));          // sv_1dpool_boundary
+        h[0] = __dadd_rn(b[3], __dmul_rn(A.lc, __dadd_rn(h[1], -b[2])));
+        e[r - 1] = __dadd_rn(b[5], __dmul_rn(A.lc, __dadd_rn(e[r - 2], -b[4])));
+        h[r - 1] = __dadd_rn(b[7], __dmul_rn(A.lc, __dadd_rn(h[r - 2], -b[6])));
+        b[0] = e[0]; b[1] = e[1]; b[2] = h[0]; b[3] = h[1];                          // _boundary_copy
+        b[4] = e[r - 1]; b[5] = e[r - 2]; b[6] = h[r - 1]; b[7] = h[r - 2];
+        e[0] = (s < A.nwave) ? A.wave[s] : 0.0;                                        // _apply_source
     }
     __syncthreads();
-    if (tid == 0) *A.step = s + 1;
+    for (int i = tid; i < r - 1; i += nt)               // sv_1dpool_ystep_h
+        h[i] = __dadd_rn(h[i], __dmul_rn(A.chh, __dadd_rn(e[i], -e[i + 1])));
 }
 
-__global__ void aux_step_kernel(const DevAux A) { aux_step_body(A); }
-
-__global__ void aux_step_batch(const DevAux *A) { aux_step_body(A[blockIdx.x]); }
-
-__global__ void probe_capture_kernel(const DevAux A)
+// the probes of step s, whose fields are behind `fields`
+__device__ __forceinline__ void probe_row(const DevAux &A, const float *const *fields, int s)
 {
-    const int s = *A.step;     // number of completed steps
-    if (s < 1 || s - 1 >= A.nsteps_planned) return;
+    if (s < 0 || s >= A.nsteps_planned) return;
     for (int q = threadIdx.x; q < A.nprobes * 6; q += blockDim.x) {
-        int p = q / 6, comp = q % 6;
-        A.probe_out[((size_t)p * A.nsteps_planned + (s - 1)) * 6 + comp] = ld_any(A.fields[comp], A.probe_cells[p], A.storage) * (comp >= 3 ? (double)A.ihs : 1.0);
+        const int p = q / 6, comp = q % 6;
+        A.probe_out[((size_t)p * A.nsteps_planned + s) * 6 + comp] = ld_any(fields[comp], A.probe_cells[p], A.storage) * (comp >= 3 ? (double)A.ihs : 1.0);
     }
 }
+
+__global__ void aux_line_kernel(const DevAux A)
+{
+    const int s = *A.step + A.off;
+    if (A.off >= 2) probe_row(A, A.fields, s - 2);
+    aux_line(A, s);
+}
+
+__global__ void close_steps_kernel(const DevAux A, const float *const *before)
+{
+    const int s = *A.step + A.off;   // steps done after this call
+    if (A.off >= 2) probe_row(A, before, s - 2);
+    probe_row(A, A.fields, s - 1);
+    __syncthreads();
+    if (threadIdx.x == 0) *A.step = s;
+}
+
+// batches: the probes of the previous step, the 1D grid, the step counter
+__global__ void aux_step_batch(const DevAux *Aux)
+{
+    const DevAux &A = Aux[blockIdx.x];
+    const int s = *A.step;
+    probe_row(A, A.fields, s - 1);
+    aux_line(A, s);
+    __syncthreads();
+    if (threadIdx.x == 0) *A.step = s + 1;
+}
+
+// the probes of the last completed step
+__global__ void probe_capture_kernel(const DevAux A) { probe_row(A, A.fields, *A.step - 1); }
 
 // ------------------------------------------------------------ NFFF running DFT
 
@@ -287,7 +303,7 @@ template <class S>
 __device__ __forceinline__ void nfff_sample_cell(const DevNfff &N, int s)
 {
     if (N.ns <= 0 || N.nfreq <= 0 || s >= N.ns) return;
-    const int step = *N.step - 1;
+    const int step = *N.step + N.off;
     if (step < 0) return;
     const size_t ns = (size_t)N.ns;
     const int64_t c = N.cell[s];
@@ -314,7 +330,7 @@ template <class S>
 __device__ __forceinline__ void nfff_fold_full_ring(const DevNfff &N, int s)
 {
     if (N.ns <= 0 || N.nfreq <= 0) return;
-    const int step = *N.step - 1;
+    const int step = *N.step + N.off;
     if (step < 0 || step % NFFF_RING != NFFF_RING - 1) return;
     __shared__ double2 tw[NFFF_RING * NFFF_TW_MAXF];
     const bool table = N.nfreq <= NFFF_TW_MAXF;
@@ -465,7 +481,7 @@ __global__ void nfff_series_kernel(const DevNfffSeries S)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= S.ns) return;
-    const int step = *S.step - 1;
+    const int step = *S.step + S.off;
     const double C0 = 299792458.0, PI = 3.14159265358979323846;
     const double dx = S.dx, dt = S.dt;
     const int fc = S.face[s];
@@ -569,7 +585,12 @@ void launch_unpack(int storage, int hsz, const float *field, size_t off, void *h
     else unpack_t<float>(hsz, field, off, host, n, scale, st);
 }
 
-void launch_aux_step(const DevAux &a, cudaStream_t st) { aux_step_kernel<<<1, 1024, 0, st>>>(a); }
+void launch_aux_line(const DevAux &a, cudaStream_t st) { aux_line_kernel<<<1, 1024, 0, st>>>(a); }
+
+void launch_close_steps(const DevAux &a, const float *const *before, cudaStream_t st)
+{
+    close_steps_kernel<<<1, 256, 0, st>>>(a, before);
+}
 
 void launch_probe_capture(const DevAux &a, cudaStream_t st) { probe_capture_kernel<<<1, 256, 0, st>>>(a); }
 

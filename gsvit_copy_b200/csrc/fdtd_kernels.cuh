@@ -15,6 +15,7 @@ struct DevAux {                 // 1D auxiliary grid of the TSF source (1dpool.c
     double ce, chh;             // (1/eps)*dt/(EPS0*dx1) and (1/mu)*dt/(MU0*dx1)
     double lc;                  // Liao factor (dt*c - dx1)/(dt*c + dx1)
     int *step;                  // device step counter
+    int off;                    // steps since the counter was last advanced (aux_line, close_steps)
     // probes of the previous step
     int nprobes;
     const int64_t *probe_cells;
@@ -39,12 +40,16 @@ struct DevNfff {
     float *ring;                // NFFF_RING steps of raw samples [(slot*9 + 3a + r)*ns + s], r: E(c), E(c+st), E(c-st);
                                 // FP32 elements (FP64 for FDTD_STORE_F64 plans)
     const double *omega_dt;     // nfreq
-    const int *step;            // device step counter (already advanced)
+    const int *step;            // device step counter; the step sampled is *step + off
+    int off;
     double inv2dx;
     int storage;                // FDTD_STORE_* of the fields
 };
 
-void launch_aux_step(const DevAux &a, cudaStream_t st);
+// the 1D grid step of step *a.step + a.off; with a.off >= 2 also the probes of two steps before, from a.fields
+void launch_aux_line(const DevAux &a, cudaStream_t st);
+// the end of a call of a.off steps: probes of its last step (a.fields) and of the one before (`before`), step counter
+void launch_close_steps(const DevAux &a, const float *const *before, cudaStream_t st);
 
 // Batched forms: one launch covers many plans whose per-plan parameters are
 // device tables (of this step's parity), indexed by the plan number.
@@ -92,7 +97,8 @@ struct DevNfffSeries {
     const int32_t *istart;      // npoints
     const float *const *e;      // 3 E field pointers (the set written by this step)
     double *series;             // [(p*3 + c)*ndata + m]
-    const int *step;            // device step counter (already advanced)
+    const int *step;            // device step counter; the step added is *step + off
+    int off;
     double dx, dt;
     int storage;                // FDTD_STORE_* of the fields
 };
