@@ -15,11 +15,16 @@
 //      update read (the curl and the psi recursions);
 //   B: per cell of the other field, the sum of the difference adjoints of the
 //      cells whose differences contain it.
+// Memory bounds them (A and B of both half steps move 192 bytes a cell): a thread
+// takes V consecutive k cells (4, or 1 on ragged rows) of a row, its block a
+// piece of a plane.  Plans with dispersive cells take A of the E half step a
+// cell a thread.  128 x 128 x 96, 12-cell CPML: 119 -> 59 us a transposed step.
 // Gates, coefficients and operation order follow e_special / h_special.
 #include <cuda_runtime.h>
 
 #include "fdtd_adjoint.cuh"
 #include "fdtd_device.cuh"
+#include "fdtd_flat_kernels.cuh"   // vector loads and stores, slab positions
 
 namespace {
 
@@ -55,8 +60,7 @@ struct FaceT {             // one psi_E array of one face at this cell
     float ade_s;
 };
 
-template <bool ADE>
-__global__ void adj_e_a(const __grid_constant__ DevPlan P, const DevAdj A, int64_t n)
+__global__ void adj_e_a_ade(const __grid_constant__ DevPlan P, const DevAdj A, int64_t n)
 {
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
         int i, j, k;
@@ -72,7 +76,7 @@ __global__ void adj_e_a(const __grid_constant__ DevPlan P, const DevAdj A, int64
             const int64_t q = ((int64_t)(i - P.dbox[0]) * (P.dbox[3] - P.dbox[2]) + (j - P.dbox[2])) * (P.dbox[5] - P.dbox[4]) + (k - P.dbox[4]);
             for (int a = 0; a < 3; a++) { ca[a] = P.dcoef[6 * q + a]; cb[a] = P.dcoef[6 * q + 3 + a]; }
         }
-        const bool ade = ADE && (fl & CF_ADE_BRANCH);
+        const bool ade = (fl & CF_ADE_BRANCH) != 0;
         const bool comp[3] = {ade && (fl & CF_ADE_X), ade && (fl & CF_ADE_Y), ade && (fl & CF_ADE_Z)};
         const bool gd[3] = {j > 0 && k > 0, i > 0 && k > 0, i > 0 && j > 0};
         float e[3] = {A.eb[0][c], A.eb[1][c], A.eb[2][c]};
@@ -162,7 +166,7 @@ __global__ void adj_e_a(const __grid_constant__ DevPlan P, const DevAdj A, int64
         // adjoint of the ADE value of the dispersive components: u = its own
         // adjoint plus what the state recursions read from it
         float u[3] = {0.f, 0.f, 0.f};
-        if (ADE && ade) {
+        if (ade) {
             const DevAde &Ad = P.ade[__float_as_int(c2.z)];
             for (int a = 0; a < 3; a++) {
                 if (!comp[a]) continue;
@@ -203,7 +207,7 @@ __global__ void adj_e_a(const __grid_constant__ DevPlan P, const DevAdj A, int64
                 e[a] = ca[a] * e[a];
             }
         }
-        if (ADE && ade) {
+        if (ade) {
             const DevAde &Ad = P.ade[__float_as_int(c2.z)];
             for (int a = 0; a < 3; a++) {
                 if (!comp[a]) continue;
@@ -240,123 +244,316 @@ __global__ void adj_e_a(const __grid_constant__ DevPlan P, const DevAdj A, int64
     }
 }
 
-// ---- E half step: B -- H adjoints from the backward-difference adjoints
-__global__ void adj_e_b(const __grid_constant__ DevPlan P, const DevAdj A, int64_t n)
+// ---- the group of a thread: V cells from k of row j, plane i
+
+struct AdjRows {
+    int nk;            // groups a row
+    unsigned mk;       // division by nk (flat_div)
+    int sk;
+};
+
+template <int V>
+__device__ __forceinline__ bool adj_group(const DevPlan &P, const AdjRows &W, int &j, int &k)
 {
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-        int i, j, k;
-        cell_ijk(P, c, i, j, k);
-        const bool ko = k + 1 < P.zr, jo = j + 1 < P.yr, io = i + 1 < P.xr;
-        const int64_t sj = P.sj, si = P.si;
-        float hx = A.dd[2][c] + A.dd[5][c], hy = A.dd[1][c] + A.dd[4][c], hz = A.dd[0][c] + A.dd[3][c];
-        if (ko) { hx -= A.dd[2][c + 1]; hy -= A.dd[1][c + 1]; }
-        if (jo) { hx -= A.dd[5][c + sj]; hz -= A.dd[0][c + sj]; }
-        if (io) { hy -= A.dd[4][c + si]; hz -= A.dd[3][c + si]; }
-        A.hb[0][c] += hx;
-        A.hb[1][c] += hy;
-        A.hb[2][c] += hz;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned r = flat_div(t, W.mk, W.sk);
+    j = (int)r;
+    k = V * (int)(t - r * W.nk);
+    return j < P.yr;
+}
+
+// ---- E half step: A without dispersive cells (adj_e_a_ade has the derivation)
+template <int V>
+__global__ void __launch_bounds__(128) adj_e_a(const __grid_constant__ DevPlan P, const DevAdj A, const AdjRows W)
+{
+    int j, k;
+    if (!adj_group<V>(P, W, j, k)) return;
+    const int xr = P.xr, yr = P.yr, zr = P.zr;
+    const float dx = P.dx, idx_ = 1.0f / P.dx;
+    const float4 *cl = reinterpret_cast<const float4 *>(P.classes);
+    for (int i = blockIdx.y; i < xr; i += gridDim.y) {
+        const int64_t c0 = (int64_t)i * P.si + (int64_t)j * P.sj + k;
+        float e[3][V], d[6][V], ca[3][V], cb[3][V];
+        unsigned fl[V];
+#pragma unroll
+        for (int a = 0; a < 3; a++) ldv<float, V>(e[a], A.eb[a], c0);
+        const uint32_t cw = class_word<V>(P, i, j, k);
+        ECoef<float> C;
+#pragma unroll
+        for (int c = 0; c < V; c++) {
+            if (c == 0 || !one_class<V>(cw) || (C.fl & CF_DESIGN)) ecoef<float>(P, cl, (cw >> (8 * c)) & 0xff, i, j, k + c, C);
+            fl[c] = C.fl;
+#pragma unroll
+            for (int a = 0; a < 3; a++) { ca[a][c] = C.ca[a]; cb[a][c] = C.cb[a]; }
+        }
+#pragma unroll
+        for (int q = 0; q < 6; q++)
+#pragma unroll
+            for (int c = 0; c < V; c++) d[q][c] = 0.f;
+        const bool zij = (P.cp_on[X0] && i == 0) || (P.cp_on[Y0] && j == 0), kz0 = P.cp_on[Z0] != 0;
+        bool m[V];
+        // psi_E (second update and its correction) of the faces, x then y then z
+        auto face = [&](int f, int64_t q, bool vec, const float (&be)[V], const float (&ce)[V], int r, int comp, float s, int dif) {
+            float p[V];
+            ldpsi<float, V>(p, A.pe[f][r], q, vec, m, 1.f);
+#pragma unroll
+            for (int c = 0; c < V; c++) {
+                if (!m[c]) continue;
+                const float l2 = p[c] + s * dx * cb[comp][c] * e[comp][c];
+                p[c] = be[c] * l2;
+                d[dif][c] += ce[c] * idx_ * l2;
+            }
+            stpsi<float, V>(A.pe[f][r], q, vec, m, 1.f, p, 0, 0);
+        };
+        if (!zij) {
+            float be[V], ce[V];
+            auto one = [&](int f, int pos) {
+#pragma unroll
+                for (int c = 0; c < V; c++) {
+                    m[c] = !(k + c == 0);
+                    be[c] = __ldg(P.be[f] + pos);
+                    ce[c] = __ldg(P.ce[f] + pos);
+                }
+            };
+            const Slab X = slab_of(P, 0, i, xr), Y = slab_of(P, 1, j, yr);
+            if (P.cp_on[X.f] && X.pos >= 1 && j > 0) {
+                const int64_t q = ((int64_t)X.pos * yr + j) * zr + k;
+                one(X.f, X.pos);
+                face(X.f, q, true, be, ce, 0, 1, -1.f, 3);
+                face(X.f, q, true, be, ce, 1, 2, +1.f, 4);
+            }
+            if (P.cp_on[Y.f] && Y.pos >= 1 && i > 0) {
+                const int64_t q = ((int64_t)i * Y.d + Y.pos) * zr + k;
+                one(Y.f, Y.pos);
+                face(Y.f, q, true, be, ce, 0, 0, +1.f, 0);
+                face(Y.f, q, true, be, ce, 1, 2, -1.f, 5);
+            }
+            if (i > 0 && j > 0)
+                for (int f = Z0; f <= ZN; f++) {
+                    if (!P.cp_on[f]) continue;
+                    const int dep = P.cp_d[f], pos = f == Z0 ? k : k - (zr - dep);
+                    bool any = false;
+#pragma unroll
+                    for (int c = 0; c < V; c++) {
+                        m[c] = pos + c >= 1 && pos + c < dep && !(kz0 && k + c == 0);
+                        any = any || m[c];
+                    }
+                    if (!any) continue;
+                    const bool vec = V == 1 || dep % V == 0;
+                    const int64_t q = ((int64_t)i * yr + j) * dep + pos;
+                    ldtab<float, V>(be, P.be[f], pos, vec, m);
+                    ldtab<float, V>(ce, P.ce[f], pos, vec, m);
+                    face(f, q, vec, be, ce, 1, 1, +1.f, 2);
+                    face(f, q, vec, be, ce, 0, 0, -1.f, 1);
+                }
+        }
+        const float ikx = __ldg(P.ike[0] + i), iky = __ldg(P.ike[1] + j);
+        float ikz[V];
+        ldaxis<float, V>(ikz, P.ike[2], k);
+#pragma unroll
+        for (int c = 0; c < V; c++) {
+            const bool kz = k + c == 0, zero = zij || (kz && kz0);
+            const bool gd[3] = {j > 0 && !kz, i > 0 && !kz, i > 0 && j > 0};
+            const unsigned pm[3] = {CF_PEC_X, CF_PEC_Y, CF_PEC_Z};
+            float w[3];
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                if (zero || (fl[c] & pm[a])) e[a][c] = 0.f;
+                w[a] = 0.f;
+                if (!zero && gd[a]) {
+                    w[a] = cb[a][c] * e[a][c];
+                    e[a][c] = ca[a][c] * e[a][c];
+                }
+            }
+            // curl x = dhz_j iky - dhy_k ikz, curl y = dhx_k ikz - dhz_i ikx, curl z = dhy_i ikx - dhx_j iky
+            d[0][c] += w[0] * iky;
+            d[1][c] -= w[0] * ikz[c];
+            d[2][c] += w[1] * ikz[c];
+            d[3][c] -= w[1] * ikx;
+            d[4][c] += w[2] * ikx;
+            d[5][c] -= w[2] * iky;
+        }
+#pragma unroll
+        for (int a = 0; a < 3; a++) stv<float, V>(A.eb[a], c0, e[a], 1.f, 0, 0);
+#pragma unroll
+        for (int q = 0; q < 6; q++) stv<float, V>(A.dd[q], c0, d[q], 1.f, 0, 0);
+    }
+}
+
+// ---- E half step: B -- H adjoints from the backward-difference adjoints
+template <int V>
+__global__ void __launch_bounds__(128) adj_e_b(const __grid_constant__ DevPlan P, const DevAdj A, const AdjRows W)
+{
+    int j, k;
+    if (!adj_group<V>(P, W, j, k)) return;
+    const bool ko = k + V < P.zr, jo = j + 1 < P.yr;
+    for (int i = blockIdx.y; i < P.xr; i += gridDim.y) {
+        const int64_t c0 = (int64_t)i * P.si + (int64_t)j * P.sj + k;
+        const bool io = i + 1 < P.xr;
+        float d[6][V], h[3][V], d0j[V] = {}, d5j[V] = {}, d3i[V] = {}, d4i[V] = {};
+#pragma unroll
+        for (int q = 0; q < 6; q++) ldv<float, V>(d[q], A.dd[q], c0);
+#pragma unroll
+        for (int a = 0; a < 3; a++) ldv<float, V>(h[a], A.hb[a], c0);
+        if (jo) { ldv<float, V>(d0j, A.dd[0], c0 + P.sj); ldv<float, V>(d5j, A.dd[5], c0 + P.sj); }
+        if (io) { ldv<float, V>(d3i, A.dd[3], c0 + P.si); ldv<float, V>(d4i, A.dd[4], c0 + P.si); }
+        const float d1k = ko ? A.dd[1][c0 + V] : 0.f, d2k = ko ? A.dd[2][c0 + V] : 0.f;
+#pragma unroll
+        for (int c = 0; c < V; c++) {
+            const float n1 = c + 1 < V ? d[1][c + 1 < V ? c + 1 : 0] : d1k, n2 = c + 1 < V ? d[2][c + 1 < V ? c + 1 : 0] : d2k;
+            h[0][c] += d[2][c] + d[5][c] - n2 - d5j[c];
+            h[1][c] += d[1][c] + d[4][c] - n1 - d4i[c];
+            h[2][c] += d[0][c] + d[3][c] - d0j[c] - d3i[c];
+        }
+#pragma unroll
+        for (int a = 0; a < 3; a++) stv<float, V>(A.hb[a], c0, h[a], 1.f, 0, 0);
     }
 }
 
 // ---- H half step: A -- adjoint of H^{n-1/2}, psi_H and the E differences
 // dd: 0 dey_k, 1 dez_j, 2 dez_i, 3 dex_k, 4 dex_j, 5 dey_i (forward differences)
-__global__ void adj_h_a(const __grid_constant__ DevPlan P, const DevAdj A, int64_t n)
+template <int V>
+__global__ void __launch_bounds__(128) adj_h_a(const __grid_constant__ DevPlan P, const DevAdj A, const AdjRows W)
 {
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-        int i, j, k;
-        cell_ijk(P, c, i, j, k);
-        const int xr = P.xr, yr = P.yr, zr = P.zr;
-        const float4 hc = reinterpret_cast<const float4 *>(P.classes)[cls_at(P, i, j, k) * 4 + 2];
-        const float da = hc.x, db = hc.y, dbdx = db * P.dx, idx_ = 1.0f / P.dx;
-        const bool il = (i == xr - 1), jl = (j == yr - 1), kl = (k == zr - 1);
-        const bool iin = (i >= 1 && i < xr - 1), jin = (j >= 1 && j < yr - 1), kin = (k >= 1 && k < zr - 1);
-        float h[3] = {A.hb[0][c], A.hb[1][c], A.hb[2][c]};
-        float d[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        const bool zero = (P.cp_on[XN] && il && jin && kin) || (P.cp_on[YN] && jl && iin && kin) || (P.cp_on[ZN] && kl && iin && jin);
-        if (zero) {
-            h[0] = h[1] = h[2] = 0.f;
-        } else {
-            // x faces: psi[1] <- dey_i (hz -= dbdx psi[1]), psi[0] <- dez_i (hy += dbdx psi[0])
-            auto xface = [&](int f, int pos, int64_t q) {
-                const float bh = P.bh[f][pos], ch = P.ch[f][pos];
-                const float t1 = A.ph[f][1][q] - dbdx * h[2], t0 = A.ph[f][0][q] + dbdx * h[1];
-                A.ph[f][1][q] = bh * t1;
-                A.ph[f][0][q] = bh * t0;
-                d[5] += ch * idx_ * t1;
-                d[2] += ch * idx_ * t0;
-            };
-            // y faces: psi[0] <- dez_j (hx -= dbdx psi[0]), psi[1] <- dex_j (hz += dbdx psi[1])
-            auto yface = [&](int f, int pos, int64_t q) {
-                const float bh = P.bh[f][pos], ch = P.ch[f][pos];
-                const float t0 = A.ph[f][0][q] - dbdx * h[0], t1 = A.ph[f][1][q] + dbdx * h[2];
-                A.ph[f][0][q] = bh * t0;
-                A.ph[f][1][q] = bh * t1;
-                d[1] += ch * idx_ * t0;
-                d[4] += ch * idx_ * t1;
-            };
-            // z faces: psi[1] <- dex_k (hy -= dbdx psi[1]), psi[0] <- dey_k (hx += dbdx psi[0])
-            auto zface = [&](int f, int pos, int64_t q) {
-                const float bh = P.bh[f][pos], ch = P.ch[f][pos];
-                const float t1 = A.ph[f][1][q] - dbdx * h[1], t0 = A.ph[f][0][q] + dbdx * h[0];
-                A.ph[f][1][q] = bh * t1;
-                A.ph[f][0][q] = bh * t0;
-                d[3] += ch * idx_ * t1;
-                d[0] += ch * idx_ * t0;
-            };
-            if (P.cp_on[X0] && i < P.cp_d[X0] - 1 && jin && kin) xface(X0, i, ((int64_t)i * yr + j) * zr + k);
-            if (P.cp_on[Y0] && j < P.cp_d[Y0] - 1 && iin && kin) yface(Y0, j, ((int64_t)i * P.cp_d[Y0] + j) * zr + k);
-            if (P.cp_on[Z0] && k < P.cp_d[Z0] - 1 && iin && jin) zface(Z0, k, ((int64_t)i * yr + j) * P.cp_d[Z0] + k);
-            if (P.cp_on[XN] && i >= xr - P.cp_d[XN] + 1 && i < xr - 1 && jin && kin) {
-                const int ir = i - (xr - P.cp_d[XN]);
-                xface(XN, ir, ((int64_t)ir * yr + j) * zr + k);
+    int j, k;
+    if (!adj_group<V>(P, W, j, k)) return;
+    const int xr = P.xr, yr = P.yr, zr = P.zr;
+    const float idx_ = 1.0f / P.dx;
+    const float4 *cl = reinterpret_cast<const float4 *>(P.classes);
+    const bool jl = j == yr - 1, jin = j >= 1 && !jl;
+    for (int i = blockIdx.y; i < xr; i += gridDim.y) {
+        const int64_t c0 = (int64_t)i * P.si + (int64_t)j * P.sj + k;
+        const bool il = i == xr - 1, iin = i >= 1 && !il;
+        float h[3][V], d[6][V], da[V], db[V], dbdx[V];
+#pragma unroll
+        for (int a = 0; a < 3; a++) ldv<float, V>(h[a], A.hb[a], c0);
+        const uint32_t cw = class_word<V>(P, i, j, k);
+        bool kin[V], act[V], m[V];   // act: not in the planes boundary_hstep zeroes
+#pragma unroll
+        for (int c = 0; c < V; c++) {
+            Tab<float>::hcoef(P, cl, (cw >> (8 * c)) & 0xff, da[c], db[c]);
+            dbdx[c] = db[c] * P.dx;
+            const bool kl = k + c == zr - 1;
+            kin[c] = k + c >= 1 && !kl;
+            act[c] = !((P.cp_on[XN] && il && jin && kin[c]) || (P.cp_on[YN] && jl && iin && kin[c]) || (P.cp_on[ZN] && kl && iin && jin));
+#pragma unroll
+            for (int q = 0; q < 6; q++) d[q][c] = 0.f;
+        }
+        auto face = [&](int f, int64_t q, bool vec, const float (&bh)[V], const float (&ch)[V], int r, int comp, float s, int dif) {
+            float p[V];
+            ldpsi<float, V>(p, A.ph[f][r], q, vec, m, 1.f);
+#pragma unroll
+            for (int c = 0; c < V; c++) {
+                if (!m[c]) continue;
+                const float t = p[c] + s * dbdx[c] * h[comp][c];
+                p[c] = bh[c] * t;
+                d[dif][c] += ch[c] * idx_ * t;
             }
-            if (P.cp_on[YN] && j >= yr - P.cp_d[YN] + 1 && j < yr - 1 && iin && kin) {
-                const int jr = j - (yr - P.cp_d[YN]);
-                yface(YN, jr, ((int64_t)i * P.cp_d[YN] + jr) * zr + k);
+            stpsi<float, V>(A.ph[f][r], q, vec, m, 1.f, p, 0, 0);
+        };
+        {
+            float bh[V], ch[V];
+            auto one = [&](int f, int pos) {
+#pragma unroll
+                for (int c = 0; c < V; c++) {
+                    m[c] = kin[c] && act[c];
+                    bh[c] = __ldg(P.bh[f] + pos);
+                    ch[c] = __ldg(P.ch[f] + pos);
+                }
+            };
+            const Slab X = slab_of(P, 0, i, xr), Y = slab_of(P, 1, j, yr);
+            // x: psi[1] <- dey_i (hz -= dbdx psi), psi[0] <- dez_i (hy += dbdx psi)
+            if (P.cp_on[X.f] && jin && (X.f == X0 ? i < X.d - 1 : X.pos >= 1 && !il)) {
+                const int64_t q = ((int64_t)X.pos * yr + j) * zr + k;
+                one(X.f, X.pos);
+                face(X.f, q, true, bh, ch, 1, 2, -1.f, 5);
+                face(X.f, q, true, bh, ch, 0, 1, +1.f, 2);
             }
-            if (P.cp_on[ZN] && k >= zr - P.cp_d[ZN] + 1 && k < zr - 1 && iin && jin) {
-                const int kr = k - (zr - P.cp_d[ZN]);
-                zface(ZN, kr, ((int64_t)i * yr + j) * P.cp_d[ZN] + kr);
+            // y: psi[0] <- dez_j (hx -= dbdx psi), psi[1] <- dex_j (hz += dbdx psi)
+            if (P.cp_on[Y.f] && iin && (Y.f == Y0 ? j < Y.d - 1 : Y.pos >= 1 && !jl)) {
+                const int64_t q = ((int64_t)i * Y.d + Y.pos) * zr + k;
+                one(Y.f, Y.pos);
+                face(Y.f, q, true, bh, ch, 0, 0, -1.f, 1);
+                face(Y.f, q, true, bh, ch, 1, 2, +1.f, 4);
             }
-            const float ikx = P.ikh[0][i], iky = P.ikh[1][j], ikz = P.ikh[2][k];
+            // z: psi[1] <- dex_k (hy -= dbdx psi), psi[0] <- dey_k (hx += dbdx psi)
+            if (iin && jin)
+                for (int f = Z0; f <= ZN; f++) {
+                    if (!P.cp_on[f]) continue;
+                    const int dep = P.cp_d[f], pos = f == Z0 ? k : k - (zr - dep);
+                    bool any = false;
+#pragma unroll
+                    for (int c = 0; c < V; c++) {
+                        m[c] = act[c] && (f == Z0 ? k + c < dep - 1 : pos + c >= 1 && k + c < zr - 1);
+                        any = any || m[c];
+                    }
+                    if (!any) continue;
+                    const bool vec = V == 1 || dep % V == 0;
+                    const int64_t q = ((int64_t)i * yr + j) * dep + pos;
+                    ldtab<float, V>(bh, P.bh[f], pos, vec, m);
+                    ldtab<float, V>(ch, P.ch[f], pos, vec, m);
+                    face(f, q, vec, bh, ch, 1, 1, -1.f, 3);
+                    face(f, q, vec, bh, ch, 0, 0, +1.f, 0);
+                }
+        }
+        const float ikx = __ldg(P.ikh[0] + i), iky = __ldg(P.ikh[1] + j);
+        float ikz[V];
+        ldaxis<float, V>(ikz, P.ikh[2], k);
+#pragma unroll
+        for (int c = 0; c < V; c++) {
+            const bool kl = k + c == zr - 1;
+            if (!act[c]) { h[0][c] = h[1][c] = h[2][c] = 0.f; continue; }
             if (!(jl || kl)) {   // hx += db (dey_k ikz - dez_j iky)
-                const float t = db * h[0];
-                d[0] += t * ikz;
-                d[1] -= t * iky;
-                h[0] = da * h[0];
+                const float t = db[c] * h[0][c];
+                d[0][c] += t * ikz[c];
+                d[1][c] -= t * iky;
+                h[0][c] = da[c] * h[0][c];
             }
             if (!(il || kl)) {   // hy += db (dez_i ikx - dex_k ikz)
-                const float t = db * h[1];
-                d[2] += t * ikx;
-                d[3] -= t * ikz;
-                h[1] = da * h[1];
+                const float t = db[c] * h[1][c];
+                d[2][c] += t * ikx;
+                d[3][c] -= t * ikz[c];
+                h[1][c] = da[c] * h[1][c];
             }
             if (!(il || jl)) {   // hz += db (dex_j iky - dey_i ikx)
-                const float t = db * h[2];
-                d[4] += t * iky;
-                d[5] -= t * ikx;
-                h[2] = da * h[2];
+                const float t = db[c] * h[2][c];
+                d[4][c] += t * iky;
+                d[5][c] -= t * ikx;
+                h[2][c] = da[c] * h[2][c];
             }
         }
-        for (int a = 0; a < 3; a++) A.hb[a][c] = h[a];
-        for (int q = 0; q < 6; q++) A.dd[q][c] = d[q];
+#pragma unroll
+        for (int a = 0; a < 3; a++) stv<float, V>(A.hb[a], c0, h[a], 1.f, 0, 0);
+#pragma unroll
+        for (int q = 0; q < 6; q++) stv<float, V>(A.dd[q], c0, d[q], 1.f, 0, 0);
     }
 }
 
 // ---- H half step: B -- E adjoints from the forward-difference adjoints
-__global__ void adj_h_b(const __grid_constant__ DevPlan P, const DevAdj A, int64_t n)
+template <int V>
+__global__ void __launch_bounds__(128) adj_h_b(const __grid_constant__ DevPlan P, const DevAdj A, const AdjRows W)
 {
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-        int i, j, k;
-        cell_ijk(P, c, i, j, k);
-        const int64_t sj = P.sj, si = P.si;
-        float ex = -(A.dd[3][c] + A.dd[4][c]), ey = -(A.dd[0][c] + A.dd[5][c]), ez = -(A.dd[1][c] + A.dd[2][c]);
-        if (k > 0) { ex += A.dd[3][c - 1]; ey += A.dd[0][c - 1]; }
-        if (j > 0) { ex += A.dd[4][c - sj]; ez += A.dd[1][c - sj]; }
-        if (i > 0) { ey += A.dd[5][c - si]; ez += A.dd[2][c - si]; }
-        A.eb[0][c] += ex;
-        A.eb[1][c] += ey;
-        A.eb[2][c] += ez;
+    int j, k;
+    if (!adj_group<V>(P, W, j, k)) return;
+    for (int i = blockIdx.y; i < P.xr; i += gridDim.y) {
+        const int64_t c0 = (int64_t)i * P.si + (int64_t)j * P.sj + k;
+        float d[6][V], e[3][V], d4j[V] = {}, d1j[V] = {}, d5i[V] = {}, d2i[V] = {};
+#pragma unroll
+        for (int q = 0; q < 6; q++) ldv<float, V>(d[q], A.dd[q], c0);
+#pragma unroll
+        for (int a = 0; a < 3; a++) ldv<float, V>(e[a], A.eb[a], c0);
+        if (j > 0) { ldv<float, V>(d4j, A.dd[4], c0 - P.sj); ldv<float, V>(d1j, A.dd[1], c0 - P.sj); }
+        if (i > 0) { ldv<float, V>(d5i, A.dd[5], c0 - P.si); ldv<float, V>(d2i, A.dd[2], c0 - P.si); }
+        const float d3k = k > 0 ? A.dd[3][c0 - 1] : 0.f, d0k = k > 0 ? A.dd[0][c0 - 1] : 0.f;
+#pragma unroll
+        for (int c = 0; c < V; c++) {
+            const float n3 = c ? d[3][c > 0 ? c - 1 : 0] : d3k, n0 = c ? d[0][c > 0 ? c - 1 : 0] : d0k;
+            e[0][c] += n3 + d4j[c] - (d[3][c] + d[4][c]);
+            e[1][c] += n0 + d5i[c] - (d[0][c] + d[5][c]);
+            e[2][c] += d1j[c] + d2i[c] - (d[1][c] + d[2][c]);
+        }
+#pragma unroll
+        for (int a = 0; a < 3; a++) stv<float, V>(A.eb[a], c0, e[a], 1.f, 0, 0);
     }
 }
 
@@ -471,19 +668,53 @@ int grid_for(int64_t n)
 
 }  // namespace
 
+namespace {
+
+// one thread a group over (row groups, planes)
+AdjRows adj_rows(const DevPlan &p, int V, dim3 *grid)
+{
+    AdjRows w;
+    w.nk = p.zr / V;
+    flat_magic((unsigned)w.nk, &w.mk, &w.sk);
+    *grid = dim3((unsigned)(((int64_t)w.nk * p.yr + 127) / 128), (unsigned)(p.xr < 65535 ? p.xr : 65535));
+    return w;
+}
+
+template <int V>
+void adjoint_e(const DevPlan &p, const DevAdj &a, cudaStream_t st)
+{
+    dim3 grid;
+    const AdjRows w = adj_rows(p, V, &grid);
+    if (p.nade > 0) {
+        const int64_t n = (int64_t)p.xr * p.yr * p.zr;
+        adj_e_a_ade<<<grid_for(n), 256, 0, st>>>(p, a, n);
+    } else {
+        adj_e_a<V><<<grid, 128, 0, st>>>(p, a, w);
+    }
+    adj_e_b<V><<<grid, 128, 0, st>>>(p, a, w);
+}
+
+template <int V>
+void adjoint_h(const DevPlan &p, const DevAdj &a, cudaStream_t st)
+{
+    dim3 grid;
+    const AdjRows w = adj_rows(p, V, &grid);
+    adj_h_a<V><<<grid, 128, 0, st>>>(p, a, w);
+    adj_h_b<V><<<grid, 128, 0, st>>>(p, a, w);
+}
+
+}  // namespace
+
 void launch_adjoint_e(const DevPlan &p, const DevAdj &a, cudaStream_t st)
 {
-    const int64_t n = (int64_t)p.xr * p.yr * p.zr;
-    if (p.nade > 0) adj_e_a<true><<<grid_for(n), 256, 0, st>>>(p, a, n);
-    else adj_e_a<false><<<grid_for(n), 256, 0, st>>>(p, a, n);
-    adj_e_b<<<grid_for(n), 256, 0, st>>>(p, a, n);
+    if (p.zr % 4 == 0) adjoint_e<4>(p, a, st);
+    else adjoint_e<1>(p, a, st);
 }
 
 void launch_adjoint_h(const DevPlan &p, const DevAdj &a, cudaStream_t st)
 {
-    const int64_t n = (int64_t)p.xr * p.yr * p.zr;
-    adj_h_a<<<grid_for(n), 256, 0, st>>>(p, a, n);
-    adj_h_b<<<grid_for(n), 256, 0, st>>>(p, a, n);
+    if (p.zr % 4 == 0) adjoint_h<4>(p, a, st);
+    else adjoint_h<1>(p, a, st);
 }
 
 void launch_adjoint_source(const DevObjective &o, const DevAdj &a, int step, cudaStream_t st)

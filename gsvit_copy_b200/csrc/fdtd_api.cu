@@ -153,6 +153,8 @@ struct fdtd_plan {
     cudaStream_t graph_stream[2] = {nullptr, nullptr};
     std::vector<SnapItem> snap;
     double step_bytes = 0;
+    char *adj_mem = nullptr;       // scratch of the adjoint calls (Arena)
+    size_t adj_cap = 0;
 };
 
 namespace {
@@ -1375,6 +1377,7 @@ int fdtd_plan_destroy(fdtd_plan *P)
     }
     if (P->ev_fork) cudaEventDestroy(P->ev_fork);
     side_free(P);
+    if (P->adj_mem) cudaFree(P->adj_mem);
     P->mem.free_all();
     if (P->own_stream) cudaStreamDestroy(P->own_stream);
     delete P;
@@ -2279,75 +2282,103 @@ int fdtd_batch_config(const fdtd_batch *B, int *planes_per_item, int *persistent
 
 namespace {
 
-struct AdjBufs {             // adjoint state of one plan, zero-initialised
-    DevBuf mem;
-    DevAdj a;
-    ~AdjBufs() { mem.free_all(); }
+// Scratch of one adjoint call: the same calls of take() are made twice, first
+// to measure and then, after reserve(), to hand out.  One allocation instead of
+// some sixty (a gradient of 60 steps at 128 x 128 x 96 spent 30 of its 41 ms in
+// them); the plan keeps it for the next call up to KEEP bytes and gives it
+// back with itself.
+struct Arena {
+    static constexpr size_t KEEP = (size_t)2 << 30;
+    fdtd_plan *P;
+    size_t off = 0;
+    bool real = false;
+    explicit Arena(fdtd_plan *p) : P(p) {}
+    ~Arena()
+    {
+        if (P->adj_cap <= KEEP) return;
+        cudaFree(P->adj_mem);      // waits for the work that uses it
+        P->adj_mem = nullptr;
+        P->adj_cap = 0;
+    }
+    template <class T>
+    void take(T **p, size_t count)
+    {
+        if (real) *p = reinterpret_cast<T *>(P->adj_mem + off);
+        off += (count * sizeof(T) + 255) / 256 * 256;
+    }
+    cudaError_t reserve()
+    {
+        if (off > P->adj_cap) {
+            if (P->adj_mem) cudaFree(P->adj_mem);
+            P->adj_mem = nullptr;
+            P->adj_cap = 0;
+            const cudaError_t e = cudaMalloc(&P->adj_mem, off);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                return e;
+            }
+            P->adj_cap = off;
+        }
+        off = 0;
+        real = true;
+        return cudaSuccess;
+    }
 };
 
-cudaError_t adj_alloc(fdtd_plan *P, AdjBufs &B)
+// adjoint state of one plan
+void adj_take(fdtd_plan *P, Arena &m, DevAdj &a)
 {
-    std::memset(&B.a, 0, sizeof(B.a));
-    const size_t n = P->hp.n;
-    cudaError_t e;
-    for (int c = 0; c < 3; c++) {
-        if ((e = B.mem.alloc(&B.a.eb[c], n)) != cudaSuccess) return e;
-        if ((e = B.mem.alloc(&B.a.hb[c], n)) != cudaSuccess) return e;
-    }
-    for (int q = 0; q < 6; q++)
-        if ((e = B.mem.alloc(&B.a.dd[q], n)) != cudaSuccess) return e;
+    std::memset(&a, 0, sizeof(a));
     const HostPlan &hp = P->hp;
+    const size_t n = hp.n;
+    for (int c = 0; c < 3; c++) {
+        m.take(&a.eb[c], n);
+        m.take(&a.hb[c], n);
+    }
+    for (int q = 0; q < 6; q++) m.take(&a.dd[q], n);
     for (int f = 0; f < 6; f++) {
         if (!hp.cp[f].enabled) continue;
         const int dep = hp.cp[f].depth;
         const size_t cnt = (f < 2) ? (size_t)dep * hp.yr * hp.zr : (f < 4) ? (size_t)hp.xr * dep * hp.zr : (size_t)hp.xr * hp.yr * dep;
         for (int q = 0; q < 2; q++) {
-            if ((e = B.mem.alloc(&B.a.pe[f][q], cnt)) != cudaSuccess) return e;
-            if ((e = B.mem.alloc(&B.a.ph[f][q], cnt)) != cudaSuccess) return e;
+            m.take(&a.pe[f][q], cnt);
+            m.take(&a.ph[f][q], cnt);
         }
     }
     if (hp.has_ade)
         for (int c = 0; c < 3; c++) {
-            if ((e = B.mem.alloc(&B.a.ep[c], n)) != cudaSuccess) return e;
-            if ((e = B.mem.alloc(&B.a.q[c], n)) != cudaSuccess) return e;
-            for (int m = 0; m < hp.maxpoles; m++) {
-                if ((e = B.mem.alloc(&B.a.pc[c][m], n)) != cudaSuccess) return e;
-                if ((e = B.mem.alloc(&B.a.qc[c][m], n)) != cudaSuccess) return e;
+            m.take(&a.ep[c], n);
+            m.take(&a.q[c], n);
+            for (int k = 0; k < hp.maxpoles; k++) {
+                m.take(&a.pc[c][k], n);
+                m.take(&a.qc[c][k], n);
             }
         }
-    return cudaSuccess;
 }
 
 // transpose of the step with index `step`: the objective's dJ/dE of that step,
 // the design accumulation, then the E and H half steps in reverse order
-void adj_step_back(fdtd_plan *P, AdjBufs &B, const DevObjective *obj, int step, const DevGrad *g, int slot)
+void adj_step_back(fdtd_plan *P, const DevAdj &a, const DevObjective *obj, int step, const DevGrad *g, int slot)
 {
-    if (obj) launch_adjoint_source(*obj, B.a, step, P->stream);
-    if (g) launch_design_accumulate(B.a, P->dp, *g, slot, P->stream);
-    launch_adjoint_e(P->dp, B.a, P->stream);
-    launch_adjoint_h(P->dp, B.a, P->stream);
+    if (obj) launch_adjoint_source(*obj, a, step, P->stream);
+    if (g) launch_design_accumulate(a, P->dp, *g, slot, P->stream);
+    launch_adjoint_e(P->dp, a, P->stream);
+    launch_adjoint_h(P->dp, a, P->stream);
 }
 
 struct DevCheckpoints {      // device copies of the stepping state
-    DevBuf mem;
-    size_t bytes = 0;
     std::vector<unsigned char *> slot;
     std::vector<int> cur, step;
-    ~DevCheckpoints() { mem.free_all(); }
 };
 
-cudaError_t ckpt_alloc(fdtd_plan *P, DevCheckpoints &K, int nslots)
+void ckpt_take(fdtd_plan *P, Arena &m, DevCheckpoints &K, int nslots)
 {
-    for (auto &s : P->snap) K.bytes += (s.bytes + 255) / 256 * 256;
-    for (int q = 0; q < nslots; q++) {
-        unsigned char *p;
-        cudaError_t e = K.mem.alloc(&p, K.bytes);
-        if (e != cudaSuccess) return e;
-        K.slot.push_back(p);
-    }
+    size_t bytes = 0;
+    for (auto &s : P->snap) bytes += (s.bytes + 255) / 256 * 256;
+    K.slot.resize(nslots);
+    for (auto &p : K.slot) m.take(&p, bytes);
     K.cur.assign(nslots, 0);
     K.step.assign(nslots, 0);
-    return cudaSuccess;
 }
 
 cudaError_t ckpt_save(fdtd_plan *P, DevCheckpoints &K, int q)
@@ -2438,18 +2469,24 @@ int fdtd_adjoint_transpose(fdtd_plan *P, int nsteps, double *const comps[6])
     int rc = check_adjoint_plan(P);
     if (rc != FDTD_OK) return rc;
     CK(cudaSetDevice(P->device));
-    AdjBufs B;
-    CK(adj_alloc(P, B));
+    DevAdj a;
+    Arena m(P);
+    adj_take(P, m, a);
+    const size_t total = m.off;
+    CK(m.reserve());
+    adj_take(P, m, a);
+    CK(cudaMemsetAsync(P->adj_mem, 0, total, P->stream));
+    CK(cudaStreamSynchronize(P->stream));
     const size_t n = P->hp.n;
     std::vector<float> tmp(n);
     for (int c = 0; c < 6; c++) {
         for (size_t q = 0; q < n; q++) tmp[q] = (float)comps[c][q];
-        CK(cudaMemcpy(c < 3 ? B.a.eb[c] : B.a.hb[c - 3], tmp.data(), n * 4, cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(c < 3 ? a.eb[c] : a.hb[c - 3], tmp.data(), n * 4, cudaMemcpyHostToDevice));
     }
-    for (int s = 0; s < nsteps; s++) adj_step_back(P, B, nullptr, 0, nullptr, 0);
+    for (int s = 0; s < nsteps; s++) adj_step_back(P, a, nullptr, 0, nullptr, 0);
     CK(cudaGetLastError());
     for (int c = 0; c < 6; c++) {
-        CK(cudaMemcpyAsync(tmp.data(), c < 3 ? B.a.eb[c] : B.a.hb[c - 3], n * 4, cudaMemcpyDeviceToHost, P->stream));
+        CK(cudaMemcpyAsync(tmp.data(), c < 3 ? a.eb[c] : a.hb[c - 3], n * 4, cudaMemcpyDeviceToHost, P->stream));
         CK(cudaStreamSynchronize(P->stream));
         for (size_t q = 0; q < n; q++) comps[c][q] = (double)tmp[q];
     }
@@ -2466,11 +2503,36 @@ int fdtd_adjoint_gradient(fdtd_plan *P, const fdtd_objective *obj, int nsteps, i
     if (rc != FDTD_OK) return rc;
     CK(cudaSetDevice(P->device));
     const int K = std::min(checkpoint, nsteps), nseg = (nsteps + K - 1) / K;
+    // adjoint state and design accumulators (zeroed), objective, curls, checkpoints
     DevCheckpoints ck;
+    DevAdj adj;
+    DevGrad g;
+    for (int q = 0; q < 6; q++) g.box[q] = P->hp.abox[q];
+    g.ncell = (int64_t)(g.box[1] - g.box[0]) * (g.box[3] - g.box[2]) * (g.box[5] - g.box[4]);
+    int32_t *dpts;
+    double *dw;
+    double2 *ae, *ad;
+    const int ns = P->nf.ns;
+    size_t zeroed = 0;
+    Arena m(P);
+    auto layout = [&]() {
+        adj_take(P, m, adj);
+        m.take(&g.g, (size_t)3 * g.ncell);
+        zeroed = m.off;
+        m.take(&dpts, (size_t)obj->npoints);
+        m.take(&dw, (size_t)obj->npoints);
+        m.take(&ae, (size_t)3 * ns);
+        m.take(&ad, (size_t)3 * ns);
+        m.take(&g.curl, (size_t)K * 3 * g.ncell);
+        ckpt_take(P, m, ck, nseg + 1);
+    };
+    layout();
     {
-        cudaError_t e = ckpt_alloc(P, ck, nseg + 1);
-        if (e != cudaSuccess) return fail(FDTD_E_NOMEM, std::string("adjoint checkpoints: ") + cudaGetErrorString(e));
+        const cudaError_t e = m.reserve();
+        if (e != cudaSuccess) return fail(FDTD_E_NOMEM, std::string("adjoint checkpoints and state: ") + cudaGetErrorString(e));
     }
+    layout();
+    CK(cudaMemsetAsync(P->adj_mem, 0, zeroed, P->stream));
     // forward pass with a checkpoint at the start of every segment
     for (int seg = 0; seg < nseg; seg++) {
         const int len = std::min(K, nsteps - seg * K);
@@ -2485,17 +2547,8 @@ int fdtd_adjoint_gradient(fdtd_plan *P, const fdtd_objective *obj, int nsteps, i
     CK(cudaGetLastError());
     rc = objective_from_spectrum(P, obj, J);
     if (rc != FDTD_OK) return rc;
-    // objective weights, adjoint state, design accumulators
-    DevBuf mem;
-    struct Free { DevBuf &m; ~Free() { m.free_all(); } } guard{mem};
-    int32_t *dpts;
-    double *dw;
-    double2 *ae, *ad;
-    const int ns = P->nf.ns;
-    CK(upload(mem, &dpts, obj->points, (size_t)obj->npoints));
-    CK(upload(mem, &dw, obj->weights, (size_t)obj->npoints));
-    CK(mem.alloc(&ae, (size_t)3 * ns));
-    CK(mem.alloc(&ad, (size_t)3 * ns));
+    CK(cudaMemcpyAsync(dpts, obj->points, (size_t)obj->npoints * sizeof(int32_t), cudaMemcpyHostToDevice, P->stream));
+    CK(cudaMemcpyAsync(dw, obj->weights, (size_t)obj->npoints * sizeof(double), cudaMemcpyHostToDevice, P->stream));
     launch_objective_weights(P->ff, obj->freq, obj->npoints, dpts, dw, P->ff.out, ae, ad, P->stream);
     DevObjective o;
     o.ns = ns;
@@ -2505,16 +2558,6 @@ int fdtd_adjoint_gradient(fdtd_plan *P, const fdtd_objective *obj, int nsteps, i
     o.omega_dt = P->omega[obj->freq] * P->hp.dt;
     o.ae = ae;
     o.ad = ad;
-    DevGrad g;
-    for (int q = 0; q < 6; q++) g.box[q] = P->hp.abox[q];
-    g.ncell = (int64_t)(g.box[1] - g.box[0]) * (g.box[3] - g.box[2]) * (g.box[5] - g.box[4]);
-    CK(mem.alloc(&g.g, (size_t)3 * g.ncell));
-    {
-        cudaError_t e = mem.alloc(&g.curl, (size_t)K * 3 * g.ncell);
-        if (e != cudaSuccess) return fail(FDTD_E_NOMEM, std::string("adjoint curl buffer: ") + cudaGetErrorString(e));
-    }
-    AdjBufs B;
-    CK(adj_alloc(P, B));
     // backward: recompute each segment from its checkpoint, then its steps in reverse
     for (int seg = nseg - 1; seg >= 0; seg--) {
         const int m0 = seg * K, m1 = std::min(nsteps, m0 + K);
@@ -2523,7 +2566,7 @@ int fdtd_adjoint_gradient(fdtd_plan *P, const fdtd_objective *obj, int nsteps, i
                        [&](int in, int s) { launch_design_curl(plan_for(P, in), g, s, P->stream); });
         if (rc != FDTD_OK) return rc;
         P->host_step += m1 - m0;
-        for (int m = m1 - 1; m >= m0; m--) adj_step_back(P, B, &o, m, &g, m - m0);
+        for (int s = m1 - 1; s >= m0; s--) adj_step_back(P, adj, &o, s, &g, s - m0);
         CK(cudaGetLastError());
     }
     CK(ckpt_restore(P, ck, nseg));
