@@ -58,3 +58,18 @@ def test_point_in_a_surface_cell():
     assert rel_l2(sb[:6], sa) < 1e-12 and not np.isfinite(sb[6]).all()
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("shape,points", [((20, 18, 400), [(10, 9, 900), (10, 9, -700)]),     # cells of a CTA that arrive far apart
+                                          ((28, 26, 30), _sphere(3, 60)), ((28, 26, 30), _sphere(70, 400))],
+                         ids=["long", "near", "many"])
+def test_series(shape, points):
+    s = _scene(points, 2, shape=shape, series=True)
+    g, o = Solver(s), CpuSolver(s)
+    g.step(NSTEPS)
+    o.step(NSTEPS)
+    ser, ref = g.nfff_series(), o.nfff_series()
+    assert ser.shape == ref.shape
+    assert rel_l2(ser, ref) < 1e-5, rel_l2(ser, ref)
+    g.close()
+    o.close()
