@@ -147,6 +147,8 @@ struct fdtd_plan {
     bool nfff_series = false;             // time-domain series of farfield.c, exact
     DevNfffSeries ns;
     int nfff_ndata = 0;
+    int *d_nonzero = nullptr;
+    bool one_pole = false;   // the flat E kernel steps the first pole alone (a restored state may end that)
     // graphs per parity
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     int graph_steps = 0;
@@ -198,6 +200,9 @@ DevPlan plan_for(const fdtd_plan *P, int in)
 }
 
 // one launch of the tile kernel of `kind` (TILE_*) for this step's parity
+// the variant of the flat E kernel: what the dispersive state can hold
+int flat_poles(const fdtd_plan *P) { return P->one_pole ? 1 : P->hp.maxpoles; }
+
 int launch_tile_kind(fdtd_plan *P, const DevPlan &d, int in, int kind, cudaStream_t st)
 {
     const cudaError_t e = launch_tiles(kind, d, P->tmaps[kind][in], P->d_tiles[kind], P->ntiles[kind], P->d_err,
@@ -256,7 +261,7 @@ int launch_fused(fdtd_plan *P, const DevPlan &d, int in, cudaStream_t st)
         e = launch_flat_h(d, P->flat, P->fwidth, P->storage, st);
         if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("flat H launch: ") + cudaGetErrorString(e));
     }
-    e = launch_flat_e(d, P->flat, P->fwidth, P->hp.has_ade, P->hp.maxpoles, P->storage, st);
+    e = launch_flat_e(d, P->flat, P->fwidth, P->hp.has_ade, flat_poles(P), P->storage, st);
     if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("flat E launch: ") + cudaGetErrorString(e));
     return FDTD_OK;
 }
@@ -756,6 +761,7 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
     }
     HostPlan &hp = P->hp;
     if (pole_arrays && hp.has_ade) hp.maxpoles = 2;
+    P->one_pole = hp.one_pole;
     P->storage = desc->storage;
     P->esz = desc->storage == FDTD_STORE_F32 ? 4 : desc->storage == FDTD_STORE_F64 ? 8 : 2;
     const size_t esz = P->esz;
@@ -925,6 +931,7 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
     // TSF
     std::memset(&P->aux, 0, sizeof(P->aux));
     CA(P->mem.alloc(&P->d_step, 1), "step counter");
+    if (hp.one_pole) CA(P->mem.alloc(&P->d_nonzero, 1), "state check");
     P->snap.push_back({P->d_step, sizeof(int)});
     P->aux.step = P->d_step;
     d.stepc = P->d_step;
@@ -1660,9 +1667,9 @@ int fdtd_step_profile(fdtd_plan *P, int nsteps, double out[8])
                 e = launch_tiles(TILE_BULK, d, P->bmaps[in], P->d_bulk, P->nbulk, P->d_err, P->hp.has_ade, P->hp.maxpoles,
                                  P->storage, 0, st);
             if (e == cudaSuccess) e = launch_flat_h(d, P->flat_in, P->fwidth, P->storage, st);
-            if (e == cudaSuccess) e = launch_flat_e(d, P->flat_in, P->fwidth, P->hp.has_ade, P->hp.maxpoles, P->storage, st);
+            if (e == cudaSuccess) e = launch_flat_e(d, P->flat_in, P->fwidth, P->hp.has_ade, flat_poles(P), P->storage, st);
             CK(cudaEventRecord(E[2], st));
-            if (e == cudaSuccess) e = launch_flat_e(d, P->flat_sp, P->fwidth, P->hp.has_ade, P->hp.maxpoles, P->storage, st);
+            if (e == cudaSuccess) e = launch_flat_e(d, P->flat_sp, P->fwidth, P->hp.has_ade, flat_poles(P), P->storage, st);
             if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("flat step launch: ") + cudaGetErrorString(e));
         }
         CK(cudaEventRecord(E[3], st));
@@ -1829,6 +1836,21 @@ int fdtd_snapshot_restore(fdtd_plan *P, const void *host_buf, size_t bytes)
         p += s.bytes;
     }
     CK(cudaStreamSynchronize(P->stream));
+    if (P->hp.one_pole) {   // a state from elsewhere may hold what the one-pole kernel takes for zero
+        const DevPlan &d = P->dp;
+        const float *rest[9];
+        for (int a = 0; a < 3; a++) { rest[a] = d.q[a]; rest[3 + a] = d.pc[a][1]; rest[6 + a] = d.qc[a][1]; }
+        int nonzero = 0;
+        CK(cudaMemsetAsync(P->d_nonzero, 0, sizeof(int), P->stream));
+        for (int a = 0; a < 9; a++) launch_any_nonzero(rest[a], (int64_t)d.xr * d.si, P->hp.real64, P->d_nonzero, P->stream);
+        CK(cudaMemcpyAsync(&nonzero, P->d_nonzero, sizeof(int), cudaMemcpyDeviceToHost, P->stream));
+        CK(cudaStreamSynchronize(P->stream));
+        const bool zero = !nonzero;
+        if (zero != P->one_pole)
+            for (int s = 0; s < 2; s++)
+                if (P->graph[s]) { cudaGraphExecDestroy(P->graph[s]); P->graph[s] = nullptr; }
+        P->one_pole = zero;
+    }
     return FDTD_OK;
 }
 
@@ -1870,6 +1892,7 @@ struct fdtd_batch {
     size_t items_cap[3] = {0, 0, 0};
     int nitems[3] = {0, 0, 0}, bulk_grid[3] = {0, 0, 0}, chunk_len = 0;
     bool persistent = true;
+    int graph_poles = 2;
     FlatList fh[2];          // H blocks of the instances, by cells per thread (a whole vector, one)
     FlatList fe[3][2];       // E blocks, by variant group and cells per thread
     int width[2] = {4, 1};
@@ -1936,6 +1959,16 @@ cudaError_t batch_set_items(fdtd_batch *B, int len, bool persistent)
     return cudaSuccess;
 }
 
+// One variant of the flat E kernel for the instances with poles: the one-pole
+// variant gives the bits of the general one where it applies, so an instance
+// beside others that need the latter still gets those of its own plan.
+int batch_poles(const fdtd_batch *B)
+{
+    for (size_t q = 0; q < B->plans.size(); q++)
+        if (B->group[q] == 2 && !B->plans[q]->one_pole) return 2;
+    return 1;
+}
+
 int batch_launch_step(fdtd_batch *B, cudaStream_t st)
 {
     const int in = B->cur, n = (int)B->plans.size();
@@ -1957,7 +1990,7 @@ int batch_launch_step(fdtd_batch *B, cudaStream_t st)
                               g > 0, g == 2 ? 2 : 0, B->storage, st);
     for (int g = 0; g < 3; g++)
         for (int w = 0; w < 2 && e == cudaSuccess; w++)
-            e = launch_flat_e_batch(B->d_plans[in], B->fe[g][w], B->width[w], g > 0, g == 2 ? 2 : 0, B->storage, st);
+            e = launch_flat_e_batch(B->d_plans[in], B->fe[g][w], B->width[w], g > 0, g == 2 ? batch_poles(B) : 0, B->storage, st);
     if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("batched step launch: ") + cudaGetErrorString(e));
     if (B->max_nfff) launch_nfff_accumulate_batch(B->d_nfff[in], n, B->max_nfff, st);
     B->cur = 1 - in;
@@ -2142,10 +2175,11 @@ int fdtd_batch_step_graph(fdtd_batch *B, int nsteps, int chunk)
     CK(cudaSetDevice(B->device));
     if (chunk < 2) chunk = 2;
     chunk &= ~1;   // an even number of steps returns the ping-pong parity
-    if (B->graph_steps != chunk) {
+    if (B->graph_steps != chunk || B->graph_poles != batch_poles(B)) {
         for (int s = 0; s < 2; s++)
             if (B->graph[s]) { cudaGraphExecDestroy(B->graph[s]); B->graph[s] = nullptr; }
         B->graph_steps = chunk;
+        B->graph_poles = batch_poles(B);
     }
     int done = 0;
     while (nsteps - done >= chunk) {

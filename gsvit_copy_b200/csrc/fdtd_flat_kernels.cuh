@@ -466,11 +466,14 @@ __device__ __forceinline__ void ecoef(const DevPlan &P, const float4 *cl, int cl
     }
 }
 
+// NPOLES: 0 the Drude term alone, 2 the Drude term and both poles, 1 the first
+// pole alone (a Lorentz medium: the state of the other terms is zero and stays
+// so; 150 x 118 x 131, half of it one: 126 us a step with variant 2, 94 here).
 template <bool ADE, int NPOLES, class T, int V, int FACE, bool ONE>
 __device__ __forceinline__ void flat_e_group(const DevPlan &P, const FlatCell &g)
 {
     using R = real_t<T>;
-    constexpr bool ANY = FACE == 7, EDGE = FACE != 0;
+    constexpr bool ANY = FACE == 7, EDGE = FACE != 0, DRUDE = NPOLES != 1;
     const int i = g.i, j = g.j, k = g.k, flags = g.flags;
     const int xr = P.xr, yr = P.yr, zr = P.zr;
     const int64_t c0 = (int64_t)i * P.si + (int64_t)j * P.sj + k;
@@ -514,7 +517,7 @@ __device__ __forceinline__ void flat_e_group(const DevPlan &P, const FlatCell &g
 #pragma unroll
         for (int a = 0; a < 3; a++) {
             if (!(adem & (1u << a))) continue;
-            ldstate<R, V>(qd[a], P.q[a], c0);
+            if constexpr (DRUDE) ldstate<R, V>(qd[a], P.q[a], c0);
             ldv<T, V>(w[a], P.fout[a], c0);   // E^{n-1}: the output set before this step writes it
         }
     }
@@ -636,7 +639,7 @@ __device__ __forceinline__ void flat_e_group(const DevPlan &P, const FlatCell &g
 #pragma unroll
             for (int a = 0; a < 3; a++) {
                 const R ep = w[a][c], e0 = eo[a][c];
-                R v = fma1(c0dx, cu[a], qe, qd[a][c]);
+                R v = DRUDE ? fma1(c0dx, cu[a], qe, qd[a][c]) : fma1(c0dx, cu[a], R(0), R(0));
                 if constexpr (NPOLES > 0) v += pole[a][c];
                 v += fma1(c2, ep, c3, e0);
                 ne[a][c] = v;
@@ -668,7 +671,7 @@ __device__ __forceinline__ void flat_e_group(const DevPlan &P, const FlatCell &g
                     const auto &A = Tab<R>::ade(P, C.ade);
                     const R ep = w[a][c];
                     if (gd[a]) {
-                        R v = fma1(A.c0dx, cu[a], A.qe, qd[a][c]);
+                        R v = DRUDE ? fma1(A.c0dx, cu[a], A.qe, qd[a][c]) : fma1(A.c0dx, cu[a], R(0), R(0));
                         if constexpr (NPOLES > 0) v += pole[a][c];
                         v += fma1(A.c2, ep, A.c3, e0);
                         ne[a][c] = v;
@@ -832,7 +835,8 @@ __device__ __forceinline__ void flat_e_group(const DevPlan &P, const FlatCell &g
                 }
             }
         }
-        if (all_own) {
+        if (!DRUDE && all_own) {
+        } else if (all_own) {
             const auto &A = Tab<R>::ade(P, C.ade);
             const R ma0 = A.ma0, a2 = A.a2;
 #pragma unroll
@@ -849,7 +853,7 @@ __device__ __forceinline__ void flat_e_group(const DevPlan &P, const FlatCell &g
 #pragma unroll
                 for (int a = 0; a < 3; a++) {
                     if (!(C.fl & cm[a])) continue;
-                    qd[a][c] = fma1(A.ma0, qd[a][c], A.a2, (NPOLES == 0 ? w[a][c] : mad(R(2), eo[a][c], w[a][c])) + ne[a][c]);
+                    if constexpr (DRUDE) qd[a][c] = fma1(A.ma0, qd[a][c], A.a2, (NPOLES == 0 ? w[a][c] : mad(R(2), eo[a][c], w[a][c])) + ne[a][c]);
                     if (C.fl & pm[a]) ne[a][c] = 0;
                 }
                 ne[0][c] -= zdx[c];
@@ -857,7 +861,7 @@ __device__ __forceinline__ void flat_e_group(const DevPlan &P, const FlatCell &g
         }
 #pragma unroll
         for (int a = 0; a < 3; a++)
-            if (adem & (1u << a)) ststate<R, V>(P.q[a], c0, qd[a]);
+            if (DRUDE && (adem & (1u << a))) ststate<R, V>(P.q[a], c0, qd[a]);
     }
     // the lower E planes boundary_estep zeroes (boundary.c:522-690)
 #pragma unroll
@@ -967,6 +971,7 @@ cudaError_t flat_e_v(const DevPlan *p, const DevPlan *plans, const FlatList &l, 
 {
     if (!ade) flat_e_v<false, 0, T, V>(p, plans, l, st);
     else if (npoles == 0) flat_e_v<true, 0, T, V>(p, plans, l, st);
+    else if (npoles == 1) flat_e_v<true, 1, T, V>(p, plans, l, st);
     else flat_e_v<true, 2, T, V>(p, plans, l, st);
     return cudaGetLastError();
 }

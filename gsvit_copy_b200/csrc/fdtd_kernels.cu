@@ -154,6 +154,15 @@ __device__ __forceinline__ void probe_row(const DevAux &A, const float *const *f
     }
 }
 
+// does an array of FP32 (FP64) values hold one that is neither +0 nor -0?
+__global__ void any_nonzero_kernel(const uint32_t *p, int64_t words, int real64, int *flag)
+{
+    bool any = false;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < words; q += (int64_t)gridDim.x * blockDim.x)
+        any = any || (p[q] & (real64 && !(q & 1) ? 0xffffffffu : 0x7fffffffu));
+    if (any) *flag = 1;
+}
+
 __global__ void aux_line_kernel(const DevAux A)
 {
     const int s = *A.step + A.off;
@@ -618,6 +627,11 @@ void launch_unpack(int storage, int hsz, const float *field, size_t off, void *h
     else if (storage == FDTD_STORE_F16) unpack_t<__half>(hsz, field, off, host, n, scale, st);
     else if (storage == FDTD_STORE_BF16) unpack_t<__nv_bfloat16>(hsz, field, off, host, n, scale, st);
     else unpack_t<float>(hsz, field, off, host, n, scale, st);
+}
+
+void launch_any_nonzero(const float *p, int64_t n, int real64, int *flag, cudaStream_t st)
+{
+    any_nonzero_kernel<<<1184, 256, 0, st>>>(reinterpret_cast<const uint32_t *>(p), real64 ? 2 * n : n, real64, flag);
 }
 
 void launch_aux_line(const DevAux &a, cudaStream_t st) { aux_line_kernel<<<1, 1024, 0, st>>>(a); }

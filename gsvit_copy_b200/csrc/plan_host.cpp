@@ -369,6 +369,7 @@ int build_host_plan(const fdtd_desc *d, HostPlan *hp, std::string *err)
     // ADE coefficient sets
     std::vector<int> ade_slot(std::max(d->nmat, 1), -1);
     hp->maxpoles = 0;
+    bool first_only = true;
     for (int m = 1; m < d->nmat; m++) {
         if (d->mats[m].type != FDTD_MAT_ADE) continue;
         if ((int)hp->ades.size() >= FDTD_MAX_ADE) { *err = "too many ADE materials"; return FDTD_E_UNSUPPORTED; }
@@ -388,6 +389,9 @@ int build_host_plan(const fdtd_desc *d, HostPlan *hp, std::string *err)
             w.bp2[p] = q.ade_bp2[p]; w.bp3[p] = q.ade_bp3[p]; w.bp4[p] = q.ade_bp4[p];
             if (q.ade_bp2[p] != 0 || q.ade_bp3[p] != 0 || q.ade_bp4[p] != 0) hp->maxpoles = 2;
         }
+        if (w.a2 != 0 || w.bp2[1] != 0 || w.bp3[1] != 0 || w.bp4[1] != 0 ||
+            !std::isfinite(w.qe + w.ma0 + w.pe[1] + w.qpe[1] + w.rp[1] + w.rq[1]))
+            first_only = false;
         DevAde a;
         std::memset(&a, 0, sizeof(a));
         a.c0dx = (float)w.c0dx;
@@ -404,6 +408,7 @@ int build_host_plan(const fdtd_desc *d, HostPlan *hp, std::string *err)
         hp->ades.push_back(a);
         hp->ades64.push_back(w);
     }
+    hp->one_pole = first_only && hp->maxpoles > 0;
 
     // per-cell classes, deduplicated; thread-local tables merged afterwards
     int nthr = 1;

@@ -25,6 +25,7 @@ struct HostPlan {
     std::vector<double> dcoef64;
     bool has_ade = false;
     int maxpoles = 0;
+    bool one_pole = false;               // no dispersive class has a second pole or a Drude term
     std::vector<int8_t> bnds, sskip;     // derived maps (plan.c:5387-5416, 5298-5326)
     fdtd_cpml_face cp[6];
     std::vector<float> be[6], ce[6], bh[6], ch[6];
