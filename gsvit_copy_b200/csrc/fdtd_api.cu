@@ -261,7 +261,7 @@ int launch_fused(fdtd_plan *P, const DevPlan &d, int in, cudaStream_t st)
         e = launch_flat_h(d, P->flat, P->fwidth, P->storage, st);
         if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("flat H launch: ") + cudaGetErrorString(e));
     }
-    e = launch_flat_e(d, P->flat, P->fwidth, P->hp.has_ade, flat_poles(P), P->storage, st);
+    e = launch_flat_e(d, P->flat, P->fwidth, P->hp.has_ade, flat_poles(P), P->storage, !P->bulk_on, st);
     if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("flat E launch: ") + cudaGetErrorString(e));
     return FDTD_OK;
 }
@@ -1667,9 +1667,9 @@ int fdtd_step_profile(fdtd_plan *P, int nsteps, double out[8])
                 e = launch_tiles(TILE_BULK, d, P->bmaps[in], P->d_bulk, P->nbulk, P->d_err, P->hp.has_ade, P->hp.maxpoles,
                                  P->storage, 0, st);
             if (e == cudaSuccess) e = launch_flat_h(d, P->flat_in, P->fwidth, P->storage, st);
-            if (e == cudaSuccess) e = launch_flat_e(d, P->flat_in, P->fwidth, P->hp.has_ade, flat_poles(P), P->storage, st);
+            if (e == cudaSuccess) e = launch_flat_e(d, P->flat_in, P->fwidth, P->hp.has_ade, flat_poles(P), P->storage, false, st);
             CK(cudaEventRecord(E[2], st));
-            if (e == cudaSuccess) e = launch_flat_e(d, P->flat_sp, P->fwidth, P->hp.has_ade, flat_poles(P), P->storage, st);
+            if (e == cudaSuccess) e = launch_flat_e(d, P->flat_sp, P->fwidth, P->hp.has_ade, flat_poles(P), P->storage, false, st);
             if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("flat step launch: ") + cudaGetErrorString(e));
         }
         CK(cudaEventRecord(E[3], st));

@@ -9,7 +9,7 @@
 template <class T>
 cudaError_t flat_h_t(const DevPlan *p, const DevPlan *plans, const FlatList &l, int width, cudaStream_t st);
 template <class T>
-cudaError_t flat_e_t(const DevPlan *p, const DevPlan *plans, const FlatList &l, int width, bool ade, int npoles, cudaStream_t st);
+cudaError_t flat_e_t(const DevPlan *p, const DevPlan *plans, const FlatList &l, int width, bool ade, int npoles, bool beside_h, cudaStream_t st);
 
 int flat_width(int storage, int zr)
 {
@@ -29,13 +29,13 @@ cudaError_t flat_h(const DevPlan *p, const DevPlan *plans, const FlatList &l, in
 }
 
 cudaError_t flat_e(const DevPlan *p, const DevPlan *plans, const FlatList &l, int width, bool ade, int npoles, int storage,
-                   cudaStream_t st)
+                   bool beside_h, cudaStream_t st)
 {
     if (!l.n) return cudaSuccess;
-    if (storage == FDTD_STORE_F64) return flat_e_t<double>(p, plans, l, width, ade, npoles, st);
-    if (storage == FDTD_STORE_F16) return flat_e_t<__half>(p, plans, l, width, ade, npoles, st);
-    if (storage == FDTD_STORE_BF16) return flat_e_t<__nv_bfloat16>(p, plans, l, width, ade, npoles, st);
-    return flat_e_t<float>(p, plans, l, width, ade, npoles, st);
+    if (storage == FDTD_STORE_F64) return flat_e_t<double>(p, plans, l, width, ade, npoles, beside_h, st);
+    if (storage == FDTD_STORE_F16) return flat_e_t<__half>(p, plans, l, width, ade, npoles, beside_h, st);
+    if (storage == FDTD_STORE_BF16) return flat_e_t<__nv_bfloat16>(p, plans, l, width, ade, npoles, beside_h, st);
+    return flat_e_t<float>(p, plans, l, width, ade, npoles, beside_h, st);
 }
 
 }  // namespace
@@ -45,9 +45,10 @@ cudaError_t launch_flat_h(const DevPlan &p, const FlatList &l, int width, int st
     return flat_h(&p, nullptr, l, width, storage, st);
 }
 
-cudaError_t launch_flat_e(const DevPlan &p, const FlatList &l, int width, bool ade, int npoles, int storage, cudaStream_t st)
+cudaError_t launch_flat_e(const DevPlan &p, const FlatList &l, int width, bool ade, int npoles, int storage, bool beside_h,
+                          cudaStream_t st)
 {
-    return flat_e(&p, nullptr, l, width, ade, npoles, storage, st);
+    return flat_e(&p, nullptr, l, width, ade, npoles, storage, beside_h, st);
 }
 
 cudaError_t launch_flat_h_batch(const DevPlan *plans, const FlatList &l, int width, int storage, cudaStream_t st)
@@ -58,5 +59,5 @@ cudaError_t launch_flat_h_batch(const DevPlan *plans, const FlatList &l, int wid
 cudaError_t launch_flat_e_batch(const DevPlan *plans, const FlatList &l, int width, bool ade, int npoles, int storage,
                                 cudaStream_t st)
 {
-    return flat_e(nullptr, plans, l, width, ade, npoles, storage, st);
+    return flat_e(nullptr, plans, l, width, ade, npoles, storage, false, st);
 }

@@ -59,7 +59,9 @@ struct FlatList {
 int flat_width(int storage, int zr);
 
 cudaError_t launch_flat_h(const DevPlan &p, const FlatList &l, int width, int storage, cudaStream_t st);
-cudaError_t launch_flat_e(const DevPlan &p, const FlatList &l, int width, bool ade, int npoles, int storage, cudaStream_t st);
+// beside_h: the launch before it in `st` is the step's H kernel, beside whose last blocks E may start
+cudaError_t launch_flat_e(const DevPlan &p, const FlatList &l, int width, bool ade, int npoles, int storage, bool beside_h,
+                          cudaStream_t st);
 // many plans in one launch: plans is the device table of this step's parity
 cudaError_t launch_flat_h_batch(const DevPlan *plans, const FlatList &l, int width, int storage, cudaStream_t st);
 cudaError_t launch_flat_e_batch(const DevPlan *plans, const FlatList &l, int width, bool ade, int npoles, int storage,
