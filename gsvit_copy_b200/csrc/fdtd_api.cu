@@ -1117,8 +1117,13 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
             CA(upload(P->mem, &dtw, tw.data(), tw.size()), "far-field twiddles");
             int nsm = 148;
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-            const int ptiles = (f.npoints + 127) / 128;
-            int groups = (4 * nsm + ptiles - 1) / ptiles;
+            // groups of surface cells: blocks for whole waves at 2, 3 or 6 blocks an SM (1, 3 and 4
+            // frequencies a launch; 192^3, 4186 points: 10.3 ms at 2.1 blocks an SM, 7.0 at 6, 6.9 at 12),
+            // in partial sums of 256 MB at most where that leaves blocks for four an SM
+            const int ptiles = (f.npoints + FF_TILE - 1) / FF_TILE;
+            const size_t row = (size_t)f.npoints * f.nfreq * 3 * sizeof(double2);
+            const int least = (4 * nsm + ptiles - 1) / ptiles;
+            int groups = std::max(std::min(6 * nsm / ptiles, (int)((size_t(256) << 20) / row)), std::min(least, 6 * nsm / ptiles));
             groups = std::max(1, std::min(groups, std::max(1, (int)cell.size() / 256)));
             CA(P->mem.alloc(&part, (size_t)groups * f.npoints * f.nfreq * 3), "far-field partial sums");
             P->nf.ns = (int)cell.size();

@@ -372,99 +372,119 @@ __global__ void __launch_bounds__(128, 3) nfff_fold_batch(const DevNfff *N)
 // with r, cos(theta), a, b, c and the retarded index R = (int)(1 + r/(c dt)) of
 // farfield.c:175-405: the DFT of the reference time-domain series.
 //
-// Tiled over (far points x surface-cell groups): a CTA owns 128 far points
-// (one per thread) and one group of surface cells, staged 32 at a time in
-// shared memory with their accumulators for NF frequencies (read once per
-// CTA instead of once per point).  exp(-i omega R dt) comes from a table over
-// R; exp(+i omega istart dt), the face area and the sum over groups are
-// applied by farfield_reduce_kernel.  FP64 throughout, and FP64 arithmetic is
-// what bounds it: the factors of a cell alone (z E, (z^2 - 1) E, z D) are formed
-// when it is staged, the geometry takes one reciprocal square root, and the
-// reference's square root and division run only for the pairs whose retarded
-// index they could decide (about 190 -> 130 FP64 instructions a pair at three
-// frequencies; 192^3, 4186 points: 13.9 -> 11.7 ms).  A thread owns a far point so
-// that each staged surface cell serves the CTA's 128 points.
+// Tiled over (far points x surface-cell groups): a CTA owns 128 * FF_PTS far
+// points and one group of surface cells, staged 32 at a time in shared memory
+// with their accumulators for NF frequencies.  exp(-i omega R dt) = w comes from
+// a table over R; exp(+i omega istart dt), the face area and the sum over groups
+// are applied by farfield_reduce_kernel.  FP64 throughout.
+//
+// With z = exp(i omega dt), z^2 - 1 = 2 i sin(omega dt) z and q = 1/r a pair adds
+//   w q cos(theta) (q + i kappa) * (-z Ehat / 4 pi)  +  w q * (sgn z Dhat / 4 pi),
+// kappa = sin(omega dt) / (c dt): the factors of a cell alone are formed when it
+// is staged, and the reference's square root and division run only for pairs
+// whose retarded index they could decide.  What bounds it is reading the staged
+// cells (each read serves the thread's FF_PTS points) and the table, then FP64
+// arithmetic (192^3, 4186 points, 3 frequencies: 13.9 ms with the factors formed
+// pair by pair, 11.7 with three staged terms and a point a thread, 7.0 now).
+constexpr int FF_PTS = FF_TILE / 128;
+
 template <int NF>
 __global__ void __launch_bounds__(128) farfield_partial_kernel(const DevFarfield F, int f0)
 {
     constexpr int CH = 32;
-    // per staged cell, frequency and component: z E, (z^2 - 1) E and z D with z = exp(i omega dt)
-    __shared__ double2 sacc[CH][NF][9];
-    __shared__ double sgeo[CH][8];   // cell, outward normal, its sign in the kernel's derivative term
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = p < F.npoints;
+    __shared__ double2 sacc[CH][NF][6];   // per staged cell, frequency and component: -z Ehat / 4 pi, sgn z Dhat / 4 pi
+    __shared__ double sgeo[CH][6];        // cell, outward normal
     const int per = (F.ns + F.groups - 1) / F.groups;
     const int s0 = blockIdx.y * per, s1 = min(F.ns, s0 + per);
     const double C0 = 299792458.0, PI = 3.14159265358979323846;
     const double dt = F.dt, dx = F.dx, c0dt = C0 * dt, cells = dx / c0dt;
-    const double idx = 1.0 / dx, k4 = 1.0 / (4.0 * PI), kc = 1.0 / (4.0 * PI * C0 * 2.0 * dt);
-    double x = 0, y = 0, z = 0;
-    if (live) { x = F.points[3 * p]; y = F.points[3 * p + 1]; z = F.points[3 * p + 2]; }
-    double acc[NF][3][2];
-    for (int f = 0; f < NF; f++)
-        for (int q = 0; q < 3; q++) acc[f][q][0] = acc[f][q][1] = 0.0;
+    const double idx = 1.0 / dx, k4 = 1.0 / (4.0 * PI);
+    int pt[FF_PTS];
+    double x[FF_PTS], y[FF_PTS], z[FF_PTS], acc[FF_PTS][NF][3][2], kappa[NF];
+#pragma unroll
+    for (int u = 0; u < FF_PTS; u++) {
+        pt[u] = (blockIdx.x * FF_PTS + u) * blockDim.x + threadIdx.x;
+        const int p = min(pt[u], F.npoints - 1);   // past the end: the last point again, not stored
+        x[u] = F.points[3 * p]; y[u] = F.points[3 * p + 1]; z[u] = F.points[3 * p + 2];
+#pragma unroll
+        for (int f = 0; f < NF; f++)
+#pragma unroll
+            for (int q = 0; q < 3; q++) acc[u][f][q][0] = acc[u][f][q][1] = 0.0;
+    }
+#pragma unroll
+    for (int f = 0; f < NF; f++) kappa[f] = sin(F.omega[f0 + f] * dt) / c0dt;
     for (int base = s0; base < s1; base += CH) {
         const int n = min(CH, s1 - base);
         __syncthreads();
         for (int q = threadIdx.x; q < n; q += blockDim.x) {
             const int fc = F.face[base + q];
-            const double sg = (fc & 1) ? 1.0 : -1.0;
             for (int a = 0; a < 3; a++) {
                 sgeo[q][a] = F.cell_ijk[3 * (base + q) + a];
-                sgeo[q][3 + a] = fc / 2 == a ? sg : 0.0;   // angle(): normal of the face (farfield.c:44-54)
+                sgeo[q][3 + a] = fc / 2 == a ? ((fc & 1) ? 1.0 : -1.0) : 0.0;   // angle(): normal of the face (farfield.c:44-54)
             }
-            sgeo[q][6] = sg;
         }
         for (int t = threadIdx.x; t < n * NF * 3; t += blockDim.x) {
             const int q = t % n, fc = t / n, f = fc / 3, c = fc % 3;
             const double2 *A = F.acc + ((size_t)(f0 + f) * 6 + c) * F.ns + base + q;
             const double2 E = A[0], D = A[(size_t)3 * F.ns];
-            const double om = F.omega[f0 + f];
-            double zs, zc, z2s, z2c;
-            sincos(om * dt, &zs, &zc);
-            sincos(2.0 * om * dt, &z2s, &z2c);
-            z2c -= 1.0;
-            sacc[q][f][c] = make_double2(zc * E.x - zs * E.y, zc * E.y + zs * E.x);
-            sacc[q][f][3 + c] = make_double2(z2c * E.x - z2s * E.y, z2c * E.y + z2s * E.x);
-            sacc[q][f][6 + c] = make_double2(zc * D.x - zs * D.y, zc * D.y + zs * D.x);
+            double zs, zc;
+            sincos(F.omega[f0 + f] * dt, &zs, &zc);
+            const double kd = (F.face[base + q] & 1) ? k4 : -k4;
+            sacc[q][f][c] = make_double2(-k4 * (zc * E.x - zs * E.y), -k4 * (zc * E.y + zs * E.x));
+            sacc[q][f][3 + c] = make_double2(kd * (zc * D.x - zs * D.y), kd * (zc * D.y + zs * D.x));
         }
         __syncthreads();
-        if (!live) continue;
         for (int q = 0; q < n; q++) {
-            const double rx = x - sgeo[q][0], ry = y - sgeo[q][1], rz = z - sgeo[q][2];
-            const double d2 = rx * rx + ry * ry + rz * rz;
-            const double dot = sgeo[q][3] * rx + sgeo[q][4] * ry + sgeo[q][5] * rz;
-            // The retarded index needs the reference's square root and division
-            // only where they could round across an integer (and in the
-            // surface cell itself, where rt is no number).
-            const double irc = rsqrt(d2);
-            const double rt = 1.0 + d2 * irc * cells;
-            int R = (int)rt;
-            const double fr = rt - R, tol = rt * 8e-15;
-            if (!(fr >= tol && fr <= 1.0 - tol)) R = (int)(1.0 + sqrt(d2) * dx / c0dt);
-            R = min(R, F.ntw - 1);
-            const double ct = dot * irc, ir = irc * idx;
-            const double a = sgeo[q][6] * ir * k4;
-            const double b = -ct * k4 * ir * ir;
-            const double cp = -ct * kc * ir;
+            double ir[FF_PTS], ct[FF_PTS];
+            int R[FF_PTS];
+#pragma unroll
+            for (int u = 0; u < FF_PTS; u++) {
+                const double rx = x[u] - sgeo[q][0], ry = y[u] - sgeo[q][1], rz = z[u] - sgeo[q][2];
+                const double d2 = rx * rx + ry * ry + rz * rz;
+                const double dot = sgeo[q][3] * rx + sgeo[q][4] * ry + sgeo[q][5] * rz;
+                // The retarded index needs the reference's square root and division
+                // only where they could round across an integer (and in the
+                // surface cell itself, where rt is no number).
+                const double irc = rsqrt(d2);
+                const double rt = 1.0 + d2 * irc * cells;
+                R[u] = (int)rt;
+                const double fr = rt - R[u], tol = rt * 8e-15;
+                if (!(fr >= tol && fr <= 1.0 - tol)) R[u] = (int)(1.0 + sqrt(d2) * dx / c0dt);
+                R[u] = min(R[u], F.ntw - 1);
+                ct[u] = dot * irc;
+                ir[u] = irc * idx;
+            }
 #pragma unroll
             for (int f = 0; f < NF; f++) {
-                const double2 w = __ldg(&F.tw[(size_t)(f0 + f) * F.ntw + R]);
+                double wr[FF_PTS], wi[FF_PTS], gr[FF_PTS], gi[FF_PTS];
+#pragma unroll
+                for (int u = 0; u < FF_PTS; u++) {
+                    const double2 w = __ldg(&F.tw[(size_t)(f0 + f) * F.ntw + R[u]]);
+                    wr[u] = w.x * ir[u];
+                    wi[u] = w.y * ir[u];
+                    const double br = ct[u] * ir[u], bi = ct[u] * kappa[f];
+                    gr[u] = wr[u] * br - wi[u] * bi;
+                    gi[u] = wr[u] * bi + wi[u] * br;
+                }
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
-                    const double2 e1 = sacc[q][f][c], e2 = sacc[q][f][3 + c], d = sacc[q][f][6 + c];
-                    const double tr = b * e1.x + cp * e2.x + a * d.x;
-                    const double ti = b * e1.y + cp * e2.y + a * d.y;
-                    acc[f][c][0] += w.x * tr - w.y * ti;
-                    acc[f][c][1] += w.x * ti + w.y * tr;
+                    const double2 e = sacc[q][f][c], d = sacc[q][f][3 + c];
+#pragma unroll
+                    for (int u = 0; u < FF_PTS; u++) {
+                        acc[u][f][c][0] += gr[u] * e.x - gi[u] * e.y + wr[u] * d.x - wi[u] * d.y;
+                        acc[u][f][c][1] += gr[u] * e.y + gi[u] * e.x + wr[u] * d.y + wi[u] * d.x;
+                    }
                 }
             }
         }
     }
-    if (live)
+#pragma unroll
+    for (int u = 0; u < FF_PTS; u++) {
+        if (pt[u] >= F.npoints) continue;
         for (int f = 0; f < NF; f++)
             for (int c = 0; c < 3; c++)
-                F.part[(((size_t)blockIdx.y * F.npoints + p) * F.nfreq + f0 + f) * 3 + c] = make_double2(acc[f][c][0], acc[f][c][1]);
+                F.part[(((size_t)blockIdx.y * F.npoints + pt[u]) * F.nfreq + f0 + f) * 3 + c] = make_double2(acc[u][f][c][0], acc[u][f][c][1]);
+    }
 }
 
 // out = area * exp(+i omega istart dt) * sum over groups (fixed order)
@@ -681,7 +701,7 @@ void launch_nfff_fold_pending(const DevNfff &n, cudaStream_t st)
 void launch_farfield_finalize(const DevFarfield &f, cudaStream_t st)
 {
     if (f.npoints <= 0 || f.nfreq <= 0) return;
-    const dim3 grid((f.npoints + 127) / 128, f.groups);
+    const dim3 grid((f.npoints + FF_TILE - 1) / FF_TILE, f.groups);
     for (int f0 = 0; f0 < f.nfreq; f0 += 4) {
         switch (f.nfreq - f0) {
         case 1: farfield_partial_kernel<1><<<grid, 128, 0, st>>>(f, f0); break;

@@ -105,4 +105,5 @@ struct DevNfffSeries {
 };
 void launch_nfff_series(const DevNfffSeries &s, cudaStream_t st);
 
+constexpr int FF_TILE = 256;   // far points of a block of the far-field sum
 void launch_farfield_finalize(const DevFarfield &f, cudaStream_t st);
