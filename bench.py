@@ -51,8 +51,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, HERE)
 
 METRIC = "Gcell-updates/s"
-# steps per CUDA graph of the timed runs (fdtd_step_graph); at 512^3 the
-# replayed step is 2.70 ms against 2.75 ms launched eagerly
+# steps per CUDA graph of the timed runs (fdtd_step_graph)
 GRAPH_CHUNK = 32
 UNIT = "Gcell/s"
 # bounded CPU sample of the workload: same scene recipe at 128^3 with the far
@@ -269,7 +268,7 @@ def ncu_traffic(res, kernel="bulk_kernel"):
 
 KERNEL_NAMES = {
     "bulk": "tile_kernel, bulk layout (TMA-staged fused H+E step of the interior box)",
-    "cpml": "tile_kernel, CPML layouts (TMA-staged fused H+E step with psi, kappa and ADE-in-CPML)",
+    "cpml": "flat_h_kernel + flat_e_kernel (the cells around the interior: psi, kappa and ADE-in-CPML)",
 }
 
 
@@ -294,7 +293,7 @@ def kernel_rooflines(prof, nprof, step_bytes, step_ms, peak, peak_kind, res):
     t = ks[top]
     roofline = {"kernel": t["kernel"], "bound": "hbm", "achieved": t["achieved_gbs"], "peak": peak, "unit": "GB/s",
                 "frac": t["frac"], "peak_source": peak_kind,
-                "traffic": ncu_traffic(res, "bulk_kernel" if top == "bulk" else "cpml_tiles"),
+                "traffic": ncu_traffic(res) if top == "bulk" else None,
                 "algorithmic_bytes": t["algorithmic_bytes"], "ms_per_launch": t["ms_per_launch"],
                 "step_share": t["step_share"]}
     step_gbs = step_bytes / (step_ms * 1e-3) / 1e9

@@ -265,8 +265,8 @@ int fdtd_step(fdtd_plan *plan, int nsteps);
  * (chunk rounded down to an even number >= 2; one graph per field-set
  * parity, kept until a call with another chunk or the plan's destruction;
  * the steps past the last whole chunk run as fdtd_step).  Bitwise equal to
- * fdtd_step and the faster of the two for long runs: 2.69 against 2.75 ms
- * a step on the 512^3 rough surface.  */
+ * fdtd_step and the faster of the two for long runs: 18.8 against 24.0 us
+ * a step at 64^3, 374 against 378 at 256^3 (rough surface).  */
 int fdtd_step_graph(fdtd_plan *plan, int nsteps, int chunk);
 
 /* Same as fdtd_step, with its scratch in static device memory.  No
@@ -305,8 +305,10 @@ int fdtd_get_step(const fdtd_plan *plan, int *step);
 int fdtd_step_timed(fdtd_plan *plan, int nsteps, double *fused_ms, int *fused_launches);
 
 /* Per-kernel profile of nsteps steps (CUDA events around every launch):
- * out[0..1] = bulk kernel total ms / algorithmic bytes per launch,
- * out[2..3] = slab kernels (H+E) total ms / algorithmic bytes per launch,
+ * out[0..1] = the plain interior (bulk kernel, or the flat H and E kernels
+ * over it), total ms / algorithmic bytes per step,
+ * out[2..3] = everything around it (flat kernels or CPML tiles), total ms /
+ * algorithmic bytes per step,
  * out[4] = 1D aux grid + TSF face tables total ms, out[5] = NFFF running DFT
  * total ms, out[6] = all kernels of the steps total ms, out[7] = kernel
  * launches per step. */
@@ -344,10 +346,11 @@ int fdtd_get_nclasses(const fdtd_plan *plan, int *nclasses);
  * stepped in lockstep: each kernel of a step is one launch over all of them,
  * with per-instance parameter tables on the device (one launch per kernel
  * variant in use: no ADE, Drude, critical-point poles).  Each instance runs
- * the kernels it runs alone: the TMA tiles over its whole grid, one CTA per
- * tile of every such instance, or else a persistent bulk kernel that walks
- * the concatenated bulk work list, and the slab kernels.  Results are
- * bit-identical to the same plans stepped one by one. */
+ * the kernels it runs alone: the flat H and E kernels over one list of all
+ * instances' blocks, with a persistent bulk kernel that walks the
+ * concatenated bulk work list, or the TMA tiles over its whole grid, where a
+ * plan of its kind uses them.  Results are bit-identical to the same plans
+ * stepped one by one. */
 typedef struct fdtd_batch fdtd_batch;
 
 /* Create nplans plans from descs[0..nplans) on one device and stream.  The
