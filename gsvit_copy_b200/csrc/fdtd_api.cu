@@ -328,13 +328,15 @@ void close_steps(fdtd_plan *P, int n, cudaStream_t st)
 // surface: 30 -> 20 us a step, 256^3: 393 -> 381, 512^3: 2310 -> 2270).  Two
 // sets of TSF tables alternate.  `tab`: one set for all steps, everything in
 // order on `st` (fdtd_step_static_scratch).  `after` (if set) is called after
-// the field update of each step with its input set.
+// the field update of each step with its input set.  `sums` false leaves the
+// far-field sums alone (the adjoint's recomputed steps, whose sums the restored
+// state replaces: 128 x 128 x 96 gradient, 60 steps, 14.7 -> 14.2 ms).
 template <class F>
-int run_steps(fdtd_plan *P, int n, cudaStream_t st, const TsfTab *tab, F after)
+int run_steps(fdtd_plan *P, int n, cudaStream_t st, const TsfTab *tab, F after, bool sums = true)
 {
     if (n <= 0) return FDTD_OK;
     const bool piped = !tab;
-    const bool has_prep = P->aux.res || P->aux.nprobes, has_post = P->nfff;
+    const bool has_prep = P->aux.res || P->aux.nprobes, has_post = P->nfff && sums;
     const int c0 = P->cur;
     auto set_in = [&](int s) { return (c0 + s) & 1; };           // step s reads this set, writes the other
     auto tables = [&](int s) -> const TsfTab & { return tab ? *tab : P->tab[s & 1]; };
@@ -360,9 +362,9 @@ int run_steps(fdtd_plan *P, int n, cudaStream_t st, const TsfTab *tab, F after)
         P->cur = 1 - in;
         if (pre) CK(cudaStreamWaitEvent(st, P->ev_prep, 0));
         if (pst) CK(cudaStreamWaitEvent(st, P->ev_post, 0));
-        if (!piped) launch_nfff(P, s, 1 - in, st);
+        if (!piped && sums) launch_nfff(P, s, 1 - in, st);
     }
-    if (piped) launch_nfff(P, n - 1, P->cur, st);
+    if (piped && sums) launch_nfff(P, n - 1, P->cur, st);
     close_steps(P, n, st);
     CK(cudaGetLastError());
     return FDTD_OK;
@@ -2602,7 +2604,7 @@ int fdtd_adjoint_gradient(fdtd_plan *P, const fdtd_objective *obj, int nsteps, i
         const int m0 = seg * K, m1 = std::min(nsteps, m0 + K);
         CK(ckpt_restore(P, ck, seg));
         rc = run_steps(P, m1 - m0, P->stream, nullptr,
-                       [&](int in, int s) { launch_design_curl(plan_for(P, in), g, s, P->stream); });
+                       [&](int in, int s) { launch_design_curl(plan_for(P, in), g, s, P->stream); }, false);
         if (rc != FDTD_OK) return rc;
         P->host_step += m1 - m0;
         for (int s = m1 - 1; s >= m0; s--) adj_step_back(P, adj, &o, s, &g, s - m0);
