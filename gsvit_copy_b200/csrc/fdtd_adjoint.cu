@@ -19,7 +19,7 @@
 // takes V consecutive k cells (4, or 1 on ragged rows) of a row, its block a
 // piece of a plane.  Plans with dispersive cells take A of the E half step a
 // cell a thread.  128 x 128 x 96, 12-cell CPML: 119 -> 59 us a transposed step.
-// Gates, coefficients and operation order follow e_special / h_special.
+// Gates, coefficients and operation order follow flat_e_group / flat_h_group.
 #include <cuda_runtime.h>
 
 #include "fdtd_adjoint.cuh"
@@ -40,7 +40,7 @@ __device__ __forceinline__ void cell_ijk(const DevPlan &P, int64_t c, int &i, in
 // in cells of the dispersive branch, of the ADE state (E^{n-1}, Q, p, q)
 // dd: 0 dhz_j, 1 dhy_k, 2 dhx_k, 3 dhz_i, 4 dhy_i, 5 dhx_j (backward differences)
 //
-// Forward, per cell (e_special): the ADE value ne of the dispersive components
+// Forward, per cell (flat_e_group): the ADE value ne of the dispersive components
 // (c0dx curl + qe Q + sum(qpe q + pe p) + c2 E^{n-1} + c3 E^n where the curl
 // exists, E^n elsewhere), the CPML inside the branch (a first psi_E update,
 // psi1 = be psi0 + ce D/dx, and ne +/-= dx cba psi1), the state recursions

@@ -30,8 +30,8 @@
 // for the components its staged class word marks.
 //
 // In a CPML tile (CP = true) every 4-cell group inside the grid takes the
-// special path of fdtd_cpgroup.cuh: h_update with psi_H (written by the owner
-// only; halo copies read it) and e_special with psi_E, kappa, ADE-in-CPML,
+// special path of fdtd_cpgroup.cuh: cp_h_group with psi_H (written by the owner
+// only; halo copies read it) and cp_e_group with psi_E, kappa, ADE-in-CPML,
 // PEC and TSF, for the four cells at once with 4-vector psi and state
 // traffic.  The CPML kernels carry no plain path: their loop body stays
 // small enough for the instruction cache, and on a plain cell the special
@@ -415,7 +415,7 @@ __device__ __forceinline__ bool bulk_item(const DevPlan &P, const BulkMaps &M, c
             const float *eo[3] = {ex, ey, ez};
             float ne[3][4];
             if constexpr (CP) {
-                // the general E path (e_special: ADE with its CPML, ordinary
+                // the general E path (cp_e_group: ADE with its CPML, ordinary
                 // update with kappa, PEC, zeroed planes, psi_E, TSF E) by group
                 // (an own group lies inside the grid)
                 cp_e_group<CPF, ADE, NPOLES, T>(P, scls, sade, cw, i, j, kq, c0i, tsf_plane, ex, ey, ez, hx, hy, hz, hxj, hzj,

@@ -2,16 +2,16 @@
 // (four consecutive k cells of row j of plane i, as a thread of the TMA tile
 // kernel holds them).
 //
-// The arithmetic of h_update / e_special (fdtd_cells.cuh) cell by cell, in
+// The arithmetic of flat_h_group / flat_e_group (fdtd_flat_kernels.cuh) cell by cell, in
 // the same operation order, reorganised face by face so that memory moves as
 // 4-vectors: one face's psi pair is loaded for the four cells, updated and
 // stored before the next face's; the dispersive state of a component is one
-// vector per array.  A face of e_special does its first psi update (ADE
+// vector per array.  A face of flat_e_group does its first psi update (ADE
 // branch, corrections of the components the ADE owns) and its second
 // (corrections of the others) together: the two touch disjoint components.
 // The z0 correction of Ex, which the reference gates by the z component, is
 // the exception: a cell whose ADE owns Ex but not Ez takes it after its
-// polarisation recursion and PEC rule, as e_special does.  Faces go x, y, z,
+// polarisation recursion and PEC rule, as flat_e_group does.  Faces go x, y, z,
 // one per axis (tiles need every grid extent >= both depths + 8); the
 // reference's order x0 y0 z0 xn yn zn differs from it only for a corner
 // group on faces of both sides, by rounding.  FP32 arithmetic (tiles run
@@ -88,7 +88,7 @@ __device__ __forceinline__ void cp_prefetch_psi(const DevPlan &P, int i, int j, 
         pf(ZN, ((int64_t)i * yr + j) * P.cp_d[ZN] + max(kq - (zr - P.cp_d[ZN]), 0));
 }
 
-// H^{n+1/2} of a special group: h_update (special = true) then h_special,
+// H^{n+1/2} of a special group: the update with kappa, then psi_H,
 // for the four cells.  d*: the forward E differences of the cells; h: H^n
 // (FP32, unscaled) in, H^{n+1/2} out.  `owner` groups write psi_H.
 template <int CPF, class T>
@@ -233,7 +233,7 @@ __device__ __forceinline__ void cp_h_group(const DevPlan &P, const float4 *scls,
     }
 }
 
-// E^{n+1} of a special group: e_special for the four cells.  e*: E^n; h*:
+// E^{n+1} of a special group: flat_e_group for the four cells.  e*: E^n; h*:
 // H^{n+1/2} of the cells, hxj/hzj of row j-1, hxk0/hyk0 of cell kq-1,
 // hyim/hzim of plane i-1.  Writes psi_E and the dispersive state; returns
 // the new E in ne (before the store).  adem, aq, aep: the components owned by
