@@ -1198,9 +1198,12 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
         // want many planes: rough surface, us a step, flat alone / with the bulk
         // kernel: 64^3 30 / 97, 128^3 85 / 128, 192^3 196 / 223, 256^3 393 / 402,
         // 320^3 709 / 688, 384^3 1198 / 1090, 512^3 2699 / 2305.
-        // BF16 takes it wherever it can: it updates E from H before H is rounded,
-        // and stochastic rounding would carry that difference everywhere.
-        const double bulk_min = P->storage == FDTD_STORE_BF16 ? 0.0 : 25165824.0;
+        // 16-bit storage takes it wherever it can, and the CPML tiles below: they
+        // update E from H before H is rounded, the flat pair from the rounded H.
+        // That costs time (256^3 FP16, 64 steps and a read-back: 40.6 ms, flat alone
+        // 31.4), but E is the less exact for it, and at BF16 stochastic rounding
+        // would carry the difference everywhere.
+        const double bulk_min = esz == 2 ? 0.0 : 25165824.0;
         for (int pass = 0; pass < 2; pass++) {
             P->bulk_on = pass == 0;   // first the TMA kernel's box, then the flat kernels' plain box
             for (int ax = 0; ax < 3; ax++) {
@@ -1305,13 +1308,13 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
         // alone, kept as the CPML tiles had it where they used to run
         const bool tile_size = dmin >= 12 && (double)hp.n >= 16777216.0;
         d.axis_order = can_tile && tile_size;
-        // The CPML tiles run for large BF16 grids (as the bulk kernel above) and on
+        // The CPML tiles run for large 16-bit grids (as the bulk kernel above) and on
         // request (GSVIT_B200_TILES=1 at plan creation; 0 forces them off): the flat
         // kernels, beside the bulk kernel or alone, are faster at every size
         // (rough surface, ms a step, tiles / bulk and flat: 512^3 d16 2.65 / 2.31,
         // 256^3 d16 0.55 / 0.39, 192^3 d16 0.35 / 0.20, 64^3 d8 0.139 / 0.030).
         const char *tv = getenv("GSVIT_B200_TILES");
-        const bool want = tv ? tv[0] == '1' : P->storage == FDTD_STORE_BF16 && tile_size;
+        const bool want = tv ? tv[0] == '1' : esz == 2 && tile_size;
         P->tiles_on = can_tile && want;
         // test hook of the bounded-wait error path: every tile CTA of this plan
         // also waits, at most this many polls, on an mbarrier nothing arrives on

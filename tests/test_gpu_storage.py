@@ -9,6 +9,8 @@ Far field of the rough-surface workload at 128^3 from rest (the physical
 pulse, 4000 steps, the 91 x 181 far grid) against an FP64 run of the same
 scene: FP32 within 1e-5, FP16 within the 1e-3 storage target; BF16 misses
 that target (expected failure, reason in the test)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -47,6 +49,37 @@ def test_fields_vs_oracle(kind, storage):
     assert max(errs) < FIELD_TOL[storage], errs
     prof = g.step_profile(1)
     assert prof["bulk_bytes"] > 0, "the TMA bulk kernel did not take the interior"
+
+
+@pytest.mark.parametrize("shape,depth", [(SHAPE, 5), ((256, 256, 256), 12)], ids=["interior", "all_cells"])
+def test_f16_e_follows_from_unrounded_h(shape, depth):
+    """E of a step comes from H before its storage rounds it: in the interior of
+    any grid whose k rows are whole 16-byte vectors, and in every cell of grids
+    of 2^24 cells and 12-cell CPML.  H = 1 A/m everywhere (a step of FP16 there:
+    1e-3) and E about 0.05 V/m: one step against the FP32 plan's from the same state.
+
+    Bound of a cell: half a unit of E in FP16 (2^-11 |E|), plus 1e-4 for the four
+    H of a curl, each within a unit of FP32 (109 ohm times 4 2^-23 is 5.2e-5).  H
+    rounded to FP16 loses its update of 4e-5 A/m: 4e-3 V/m of E."""
+    rng = np.random.default_rng(8)
+    e0 = [(rng.integers(-1024, 1025, size=shape) * 2.0 ** -14).astype(np.float32) for _ in range(3)]   # FP16 numbers
+    h0 = [np.ones(shape, dtype=np.float32)] * 3
+    out = []
+    for storage in (abi.STORE_F16, abi.STORE_F32):
+        s = plan.small_scene("lintab", shape=shape, nsteps=1)
+        s.mat[:] = 0
+        s.cpml = plan.cpml_all(depth, 3, -1, 2.0, 0.02, s.dx)
+        s.tsf = s.nfff = s.probes = None
+        s.storage = storage
+        with Solver(s) as g:
+            abi.check(g.lib.fdtd_set_fields_f32(g.h, abi.EH, abi.field_ptrs([*e0, *h0], C.c_float)))
+            g.step(1)
+            out.append(g.fields(abi.E_ALL, dtype=np.float32)[:3])
+    m = depth + 4 if shape == SHAPE else 0   # the bulk box, one cell in
+    box = tuple(slice(m, n - m) for n in shape)
+    for a, b in zip(*out):
+        a, b = a[box].astype(np.float64), b[box].astype(np.float64)
+        assert (np.abs(a - b) <= 2.0 ** -11 * np.abs(b) + 1e-4).all(), np.abs(a - b).max()
 
 
 @pytest.mark.parametrize("storage", STORES)
