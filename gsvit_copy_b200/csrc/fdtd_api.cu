@@ -282,8 +282,9 @@ DevPlan plan_at(const fdtd_plan *P, int in, int off, const TsfTab &tab)
     return d;
 }
 
-// 1D TSF grid and face corrections of step `off`; the probes of step off - 2,
-// whose fields are in set `last`
+// 1D TSF grid and face corrections of step `off`; the probes of step off - 2
+// (off >= 2) or, with the first step of a call, of the last step before it,
+// whose fields are in set `last`: the caller may have set or restored them
 void launch_prep(fdtd_plan *P, int off, int last, const TsfTab &tab, cudaStream_t st)
 {
     if (!P->aux.res && !P->aux.nprobes) return;
@@ -322,6 +323,16 @@ void close_steps(fdtd_plan *P, int n, cudaStream_t st)
     launch_close_steps(a, P->d_fieldptrs[1 - P->cur], st);
 }
 
+// the probes of the last step done, from the current fields
+int final_probes(fdtd_plan *P, cudaStream_t st)
+{
+    if (P->hp.probes.empty()) return FDTD_OK;
+    DevAux a = P->aux;
+    a.fields = P->d_fieldptrs[P->cur];
+    launch_probe_capture(a, st);
+    return FDTD_OK;
+}
+
 // n steps on `st`.  Only the field updates of a step follow from the last
 // step's: its 1D grid and TSF tables are made during the step before it, and
 // the NFFF work of a step runs during the next, on two side streams (64^3 rough
@@ -334,13 +345,13 @@ void close_steps(fdtd_plan *P, int n, cudaStream_t st)
 template <class F>
 int run_steps(fdtd_plan *P, int n, cudaStream_t st, const TsfTab *tab, F after, bool sums = true)
 {
-    if (n <= 0) return FDTD_OK;
+    if (n <= 0) return final_probes(P, st);
     const bool piped = !tab;
     const bool has_prep = P->aux.res || P->aux.nprobes, has_post = P->nfff && sums;
     const int c0 = P->cur;
     auto set_in = [&](int s) { return (c0 + s) & 1; };           // step s reads this set, writes the other
     auto tables = [&](int s) -> const TsfTab & { return tab ? *tab : P->tab[s & 1]; };
-    launch_prep(P, 0, 0, tables(0), st);
+    launch_prep(P, 0, c0, tables(0), st);
     for (int s = 0; s < n; s++) {
         const bool pre = piped && has_prep && s + 1 < n, pst = piped && has_post && s > 0;
         if (pre || pst) CK(cudaEventRecord(P->ev_main, st));
@@ -373,15 +384,6 @@ int run_steps(fdtd_plan *P, int n, cudaStream_t st, const TsfTab *tab, F after, 
 int run_steps(fdtd_plan *P, int n, cudaStream_t st, const TsfTab *tab = nullptr)
 {
     return run_steps(P, n, st, tab, [](int, int) {});
-}
-
-int final_probes(fdtd_plan *P, cudaStream_t st)
-{
-    if (P->hp.probes.empty()) return FDTD_OK;
-    DevAux a = P->aux;
-    a.fields = P->d_fieldptrs[P->cur];
-    launch_probe_capture(a, st);
-    return FDTD_OK;
 }
 
 // Bulk work items of a plan: (j,k) tiles of the bulk box, planes cut into
@@ -1603,6 +1605,7 @@ int fdtd_step_graph(fdtd_plan *P, int nsteps, int chunk)
         done += chunk;
         P->host_step += chunk;
     }
+    if (done && done == nsteps) return FDTD_OK;
     const int rc = run_steps(P, nsteps - done, P->stream);
     if (rc == FDTD_OK) P->host_step += nsteps - done;
     return rc;
@@ -1624,7 +1627,7 @@ int fdtd_step_timed(fdtd_plan *P, int nsteps, double *fused_ms, int *fused_launc
     for (auto &e : ev) CK(cudaEventCreate(&e));
     for (int s = 0; s < nsteps; s++) {
         const int in = P->cur;
-        launch_prep(P, 0, 0, P->tab[0], P->stream);
+        launch_prep(P, 0, in, P->tab[0], P->stream);
         CK(cudaEventRecord(ev[2 * s], P->stream));
         int rc = launch_fused(P, plan_at(P, in, 0, P->tab[0]), in, P->stream);
         CK(cudaEventRecord(ev[2 * s + 1], P->stream));
@@ -1660,7 +1663,7 @@ int fdtd_step_profile(fdtd_plan *P, int nsteps, double out[8])
         cudaEvent_t *E = &ev[(size_t)NE * s];
         const int in = P->cur;
         CK(cudaEventRecord(E[0], st));
-        launch_prep(P, 0, 0, P->tab[0], st);
+        launch_prep(P, 0, in, P->tab[0], st);
         CK(cudaEventRecord(E[1], st));
         const DevPlan d = plan_at(P, in, 0, P->tab[0]);
         if (P->tiles_on) {

@@ -166,7 +166,7 @@ __global__ void any_nonzero_kernel(const uint32_t *p, int64_t words, int real64,
 __global__ void aux_line_kernel(const DevAux A)
 {
     const int s = *A.step + A.off;
-    if (A.off >= 2) probe_row(A, A.fields, s - 2);
+    if (A.off != 1) probe_row(A, A.fields, s - (A.off ? 2 : 1));
     aux_line(A, s);
 }
 

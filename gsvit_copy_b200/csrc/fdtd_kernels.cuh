@@ -46,8 +46,10 @@ struct DevNfff {
     int storage;                // FDTD_STORE_* of the fields
 };
 
-// the 1D grid step of step *a.step + a.off; with a.off >= 2 also the probes of two steps before, from a.fields
+// *flag = 1 if any of n FP32 (FP64) values is not zero
 void launch_any_nonzero(const float *p, int64_t n, int real64, int *flag, cudaStream_t st);
+// the 1D grid step of step *a.step + a.off; also, from a.fields, the probes of two steps before (a.off >= 2) or
+// of the step before (a.off == 0)
 void launch_aux_line(const DevAux &a, cudaStream_t st);
 // the end of a call of a.off steps: probes of its last step (a.fields) and of the one before (`before`), step counter
 void launch_close_steps(const DevAux &a, const float *const *before, cudaStream_t st);
