@@ -314,13 +314,15 @@ void launch_nfff(fdtd_plan *P, int off, int out, cudaStream_t st)
     }
 }
 
-// the end of a call of n steps: the probes of its last two, the step counter
-void close_steps(fdtd_plan *P, int n, cudaStream_t st)
+// the end of a call of n steps: the probes of its last two, the step counter.
+// `whole` false: an error ended the call inside step n, which may have written to
+// the other field set; its launch_prep has recorded the row before the last.
+void close_steps(fdtd_plan *P, int n, cudaStream_t st, bool whole = true)
 {
     DevAux a = P->aux;
     a.off = n;
     a.fields = P->d_fieldptrs[P->cur];
-    launch_close_steps(a, P->d_fieldptrs[1 - P->cur], st);
+    launch_close_steps(a, whole ? P->d_fieldptrs[1 - P->cur] : nullptr, st);
 }
 
 // the probes of the last step done, from the current fields
@@ -351,33 +353,51 @@ int run_steps(fdtd_plan *P, int n, cudaStream_t st, const TsfTab *tab, F after, 
     const int c0 = P->cur;
     auto set_in = [&](int s) { return (c0 + s) & 1; };           // step s reads this set, writes the other
     auto tables = [&](int s) -> const TsfTab & { return tab ? *tab : P->tab[s & 1]; };
-    launch_prep(P, 0, c0, tables(0), st);
-    for (int s = 0; s < n; s++) {
-        const bool pre = piped && has_prep && s + 1 < n, pst = piped && has_post && s > 0;
-        if (pre || pst) CK(cudaEventRecord(P->ev_main, st));
-        if (pre) {   // the tables of step s + 1 were last read by step s - 1
-            CK(cudaStreamWaitEvent(P->prep, P->ev_main, 0));
-            launch_prep(P, s + 1, set_in(s), tables(s + 1), P->prep);
-            CK(cudaEventRecord(P->ev_prep, P->prep));
+    int done = 0, summed = 0;   // steps whose field updates and whose NFFF work are queued
+    auto queue = [&]() {
+        launch_prep(P, 0, c0, tables(0), st);
+        for (int s = 0; s < n; s++) {
+            const bool pre = piped && has_prep && s + 1 < n, pst = piped && has_post && s > 0;
+            if (pre || pst) CK(cudaEventRecord(P->ev_main, st));
+            if (pre) {   // the tables of step s + 1 were last read by step s - 1
+                CK(cudaStreamWaitEvent(P->prep, P->ev_main, 0));
+                launch_prep(P, s + 1, set_in(s), tables(s + 1), P->prep);
+                CK(cudaEventRecord(P->ev_prep, P->prep));
+            }
+            if (pst) {   // step s - 1's fields: read by step s, written by step s + 1
+                CK(cudaStreamWaitEvent(P->post, P->ev_main, 0));
+                launch_nfff(P, s - 1, set_in(s), P->post);
+                summed = s;
+                CK(cudaEventRecord(P->ev_post, P->post));
+            }
+            if (!piped && s > 0) launch_prep(P, s, set_in(s - 1), tables(s), st);
+            const int in = set_in(s);
+            const int rc = launch_fused(P, plan_at(P, in, s, tables(s)), in, st);
+            if (rc != FDTD_OK) return rc;
+            after(in, s);
+            P->cur = 1 - in;
+            done = s + 1;
+            if (pre) CK(cudaStreamWaitEvent(st, P->ev_prep, 0));
+            if (pst) CK(cudaStreamWaitEvent(st, P->ev_post, 0));
+            if (!piped && has_post) {
+                launch_nfff(P, s, 1 - in, st);
+                summed = done;
+            }
         }
-        if (pst) {   // step s - 1's fields: read by step s, written by step s + 1
-            CK(cudaStreamWaitEvent(P->post, P->ev_main, 0));
-            launch_nfff(P, s - 1, set_in(s), P->post);
-            CK(cudaEventRecord(P->ev_post, P->post));
-        }
-        if (!piped && s > 0) launch_prep(P, s, set_in(s - 1), tables(s), st);
-        const int in = set_in(s);
-        const int rc = launch_fused(P, plan_at(P, in, s, tables(s)), in, st);
-        if (rc != FDTD_OK) return rc;
-        after(in, s);
-        P->cur = 1 - in;
-        if (pre) CK(cudaStreamWaitEvent(st, P->ev_prep, 0));
-        if (pst) CK(cudaStreamWaitEvent(st, P->ev_post, 0));
-        if (!piped && sums) launch_nfff(P, s, 1 - in, st);
-    }
-    if (piped && sums) launch_nfff(P, n - 1, P->cur, st);
-    close_steps(P, n, st);
-    CK(cudaGetLastError());
+        return (int)FDTD_OK;
+    };
+    const int rc = queue();
+    if (rc != FDTD_OK)   // `st` goes on after what the side streams were given
+        for (cudaStream_t q : {P->prep, P->post})
+            if (cudaEventRecord(P->ev_main, q) == cudaSuccess) cudaStreamWaitEvent(st, P->ev_main, 0);
+    if (has_post && summed < done) launch_nfff(P, done - 1, P->cur, st);
+    // After an error too: field set, device counter and step count go together,
+    // at the last step that was queued whole (the 1D grid may be two steps ahead).
+    close_steps(P, done, st, done == n);
+    P->host_step += done;
+    const cudaError_t e = cudaGetLastError();   // (also clears what the lines above left behind an error)
+    if (rc != FDTD_OK) return rc;
+    CK(e);
     return FDTD_OK;
 }
 
@@ -1202,8 +1222,7 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
         // 320^3 709 / 688, 384^3 1198 / 1090, 512^3 2699 / 2305.
         // 16-bit storage takes it wherever it can, and the CPML tiles below: they
         // update E from H before H is rounded, the flat pair from the rounded H.
-        // That costs time (256^3 FP16, 64 steps and a read-back: 40.6 ms, flat alone
-        // 31.4), but E is the less exact for it, and at BF16 stochastic rounding
+        // That costs time (256^3 FP16: 504 us a step, flat alone 350), but E is the less exact for it, and at BF16 stochastic rounding
         // would carry the difference everywhere.
         const double bulk_min = esz == 2 ? 0.0 : 25165824.0;
         for (int pass = 0; pass < 2; pass++) {
@@ -1500,9 +1519,7 @@ int fdtd_step(fdtd_plan *P, int nsteps)
     if (!P || nsteps < 0) return fail(FDTD_E_INVALID, "bad argument");
     if (P->failed) return refuse_failed(P);
     CK(cudaSetDevice(P->device));
-    const int rc = run_steps(P, nsteps, P->stream);
-    if (rc == FDTD_OK) P->host_step += nsteps;
-    return rc;
+    return run_steps(P, nsteps, P->stream);
 }
 
 }  // extern "C"
@@ -1563,9 +1580,7 @@ int fdtd_step_static_scratch(fdtd_plan *P, int nsteps)
             used += 2 * bytes;
         }
     }
-    rc = run_steps(P, nsteps, P->stream, &tab);
-    if (rc == FDTD_OK) P->host_step += nsteps;
-    return rc;
+    return run_steps(P, nsteps, P->stream, &tab);
 }
 
 int fdtd_step_graph(fdtd_plan *P, int nsteps, int chunk)
@@ -1582,15 +1597,17 @@ int fdtd_step_graph(fdtd_plan *P, int nsteps, int chunk)
     }
     int done = 0;
     while (nsteps - done >= chunk) {
-        const int par = P->cur;
+        const int par = P->cur, step0 = P->host_step;
         if (!P->graph[par]) {
             cudaGraph_t g;
             cudaStream_t cs = P->stream;
             CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
             const int rc = run_steps(P, chunk, cs);
+            P->cur = par;   // nothing has run yet
+            P->host_step = step0;
             if (rc != FDTD_OK) {
-                cudaStreamEndCapture(cs, &g);
-                P->cur = par;
+                if (cudaStreamEndCapture(cs, &g) == cudaSuccess && g) cudaGraphDestroy(g);
+                cudaGetLastError();
                 return rc;
             }
             CK(cudaStreamEndCapture(cs, &g));
@@ -1598,17 +1615,14 @@ int fdtd_step_graph(fdtd_plan *P, int nsteps, int chunk)
             cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
             cudaGraphDestroy(g);
             if (e != cudaSuccess) return fail(FDTD_E_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-            P->graph[par] = ge;
-            P->cur = par;   // capture advanced cur by chunk (even): unchanged
+            P->graph[par] = ge;   // (chunk is even: a replay leaves the parity)
         }
         CK(cudaGraphLaunch(P->graph[par], P->stream));
         done += chunk;
         P->host_step += chunk;
     }
     if (done && done == nsteps) return FDTD_OK;
-    const int rc = run_steps(P, nsteps - done, P->stream);
-    if (rc == FDTD_OK) P->host_step += nsteps - done;
-    return rc;
+    return run_steps(P, nsteps - done, P->stream);
 }
 
 int fdtd_get_step(const fdtd_plan *P, int *step)
@@ -2586,7 +2600,6 @@ int fdtd_adjoint_gradient(fdtd_plan *P, const fdtd_objective *obj, int nsteps, i
         CK(ckpt_save(P, ck, seg));
         rc = run_steps(P, len, P->stream);
         if (rc != FDTD_OK) return rc;
-        P->host_step += len;
     }
     CK(ckpt_save(P, ck, nseg));
     launch_nfff_fold_pending(P->nf, P->stream);
@@ -2612,7 +2625,6 @@ int fdtd_adjoint_gradient(fdtd_plan *P, const fdtd_objective *obj, int nsteps, i
         rc = run_steps(P, m1 - m0, P->stream, nullptr,
                        [&](int in, int s) { launch_design_curl(plan_for(P, in), g, s, P->stream); }, false);
         if (rc != FDTD_OK) return rc;
-        P->host_step += m1 - m0;
         for (int s = m1 - 1; s >= m0; s--) adj_step_back(P, adj, &o, s, &g, s - m0);
         CK(cudaGetLastError());
     }

@@ -173,7 +173,7 @@ __global__ void aux_line_kernel(const DevAux A)
 __global__ void close_steps_kernel(const DevAux A, const float *const *before)
 {
     const int s = *A.step + A.off;   // steps done after this call
-    if (A.off >= 2) probe_row(A, before, s - 2);
+    if (before && A.off >= 2) probe_row(A, before, s - 2);
     probe_row(A, A.fields, s - 1);
     __syncthreads();
     if (threadIdx.x == 0) *A.step = s;

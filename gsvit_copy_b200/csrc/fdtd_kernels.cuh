@@ -51,7 +51,7 @@ void launch_any_nonzero(const float *p, int64_t n, int real64, int *flag, cudaSt
 // the 1D grid step of step *a.step + a.off; also, from a.fields, the probes of two steps before (a.off >= 2) or
 // of the step before (a.off == 0)
 void launch_aux_line(const DevAux &a, cudaStream_t st);
-// the end of a call of a.off steps: probes of its last step (a.fields) and of the one before (`before`), step counter
+// the end of a call of a.off steps: probes of its last step (a.fields) and of the one before (`before`, if set), step counter
 void launch_close_steps(const DevAux &a, const float *const *before, cudaStream_t st);
 
 // Batched forms: one launch covers many plans whose per-plan parameters are
