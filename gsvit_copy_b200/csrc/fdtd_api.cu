@@ -122,7 +122,7 @@ struct fdtd_plan {
     cudaStream_t side[NTILE] = {};
     cudaEvent_t ev_fork = nullptr, ev_join[NTILE] = {};
     double tile_bytes[NTILE] = {};         // algorithmic HBM bytes per launch of each tile kind
-    char *stage = nullptr;                // staging of the host copies that change the element type
+    char *stage = nullptr;                // staging of the host copies that change the element type (get_stage)
     size_t stage_bytes = 0;
     // what a step needs and leaves (1D grid and TSF tables; NFFF) beside the steps
     // around it (run_steps)
@@ -863,9 +863,6 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
             CA(store_alloc(&P->fields[s][c], n), "field allocation");
             P->snap.push_back({P->fields[s][c], n * esz});
         }
-    // 32 MB: a copy of one chunk takes 0.6 ms, its conversion 10 us
-    P->stage_bytes = std::min<size_t>(n * 8, 32u << 20);
-    CA(P->mem.alloc(&P->stage, P->stage_bytes), "staging buffer");
     uint8_t *cls;
     {
         const int pitch = (hp.zr + 15) / 16 * 16;   // TMA row pitch must be a multiple of 16 bytes
@@ -1359,6 +1356,28 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
     return FDTD_OK;
 }
 
+// The staging buffer of the host copies, made by the first that converts: 32 MB
+// (a copy of one chunk takes 0.6 ms, its conversion 10 us), or a smaller one
+// where that cannot be had.
+int get_stage(fdtd_plan *P)
+{
+    if (P->stage) return FDTD_OK;
+    void *q = nullptr;
+    size_t want = std::min<size_t>(P->hp.n * 8, 32u << 20);
+    cudaError_t e = cudaMalloc(&q, want);
+    while (e == cudaErrorMemoryAllocation && want > (1u << 20)) {
+        want = want / 16 * 8;   // whole doubles
+        e = cudaMalloc(&q, want);
+    }
+    cudaGetLastError();
+    if (e == cudaErrorMemoryAllocation) return fail(FDTD_E_NOMEM, std::string("staging buffer: ") + cudaGetErrorString(e));
+    CK(e);
+    P->mem.ptrs.push_back(q);
+    P->stage = static_cast<char *>(q);
+    P->stage_bytes = want;
+    return FDTD_OK;
+}
+
 // Component c of the current set from / to host values of `hsz` bytes (4 float,
 // 8 double).  What the device stores as it is in host memory is copied; else
 // the device converts, a chunk at a time through the plan's staging buffer (on
@@ -1371,6 +1390,8 @@ int upload_comp(fdtd_plan *P, int c, const void *src, int hsz)
         CK(cudaMemcpyAsync(P->fields[P->cur][c], src, n * hsz, cudaMemcpyHostToDevice, P->stream));
         return FDTD_OK;
     }
+    const int rc = get_stage(P);
+    if (rc != FDTD_OK) return rc;
     const size_t step = P->stage_bytes / hsz;
     for (size_t q = 0; q < n; q += step) {
         const size_t m = std::min(step, n - q);
@@ -1388,6 +1409,8 @@ int download_comp(fdtd_plan *P, int c, void *dst, int hsz)
         CK(cudaMemcpyAsync(dst, P->fields[P->cur][c], n * hsz, cudaMemcpyDeviceToHost, P->stream));
         return FDTD_OK;
     }
+    const int rc = get_stage(P);
+    if (rc != FDTD_OK) return rc;
     const size_t step = P->stage_bytes / hsz;
     for (size_t q = 0; q < n; q += step) {
         const size_t m = std::min(step, n - q);

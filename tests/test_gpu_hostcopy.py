@@ -4,6 +4,8 @@ and their FP32 forms) convert on the device, in chunks of the staging buffer
 a grid of more than one chunk and on one smaller than a block: double to float,
 then to the storage type to nearest (H times 2^9 at 16 bits); FP64 storage keeps
 doubles."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -44,3 +46,25 @@ def test_round_trip_bits(shape, storage):
     for a, b in zip(g.fields(dtype=np.float32), want):
         assert np.array_equal(a, b.astype(np.float32))
     g.close()
+
+
+def test_staging_is_made_by_the_first_copy_that_converts():
+    """An FP32 plan read and set as FP32 holds no staging buffer (8 bytes a cell, at
+    most 32 MB; device memory comes in pieces of 2 MB)."""
+    n = 128
+    s = plan.small_scene("lintab", shape=(n, n, n), nsteps=1)
+    f = [np.zeros((n, n, n), dtype=np.float32) for _ in range(6)]
+    free = lambda: torch.cuda.mem_get_info()[0]
+    with Solver(s) as g:
+        a = free()
+        abi.check(g.lib.fdtd_set_fields_f32(g.h, abi.EH, abi.field_ptrs(f, C.c_float)))
+        g.fields(dtype=np.float32)
+        b = free()
+        g.fields()
+        c = free()
+        g.set_fields(f)
+        g.fields()
+        d = free()
+    assert b >= a - (2 << 20)
+    assert 8 * n ** 3 - (2 << 20) <= b - c <= 8 * n ** 3 + (2 << 20)
+    assert d >= c - (2 << 20)
