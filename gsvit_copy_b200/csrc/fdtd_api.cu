@@ -1378,6 +1378,21 @@ int get_stage(fdtd_plan *P)
     return FDTD_OK;
 }
 
+// `copy` of every component of `mask`.  An error returns when the copies queued
+// before it are done: the caller may free its arrays.
+template <class T, class F>
+int copy_comps(fdtd_plan *P, int mask, T *const comps[6], F copy)
+{
+    for (int c = 0; c < 6; c++) {
+        if (!(mask & (1 << c))) continue;
+        const int rc = comps[c] ? copy(c, comps[c]) : fail(FDTD_E_INVALID, "selected component pointer is NULL");
+        if (rc == FDTD_OK) continue;
+        cudaStreamSynchronize(P->stream);
+        return rc;
+    }
+    return FDTD_OK;
+}
+
 // Component c of the current set from / to host values of `hsz` bytes (4 float,
 // 8 double).  What the device stores as it is in host memory is copied; else
 // the device converts, a chunk at a time through the plan's staging buffer (on
@@ -1464,12 +1479,8 @@ int fdtd_set_fields(fdtd_plan *P, int mask, const double *const comps[6])
 {
     if (!P || !comps) return fail(FDTD_E_INVALID, "NULL argument");
     CK(cudaSetDevice(P->device));
-    for (int c = 0; c < 6; c++) {
-        if (!(mask & (1 << c))) continue;
-        if (!comps[c]) return fail(FDTD_E_INVALID, "selected component pointer is NULL");
-        int rc = upload_comp(P, c, comps[c], 8);
-        if (rc != FDTD_OK) return rc;
-    }
+    const int rc = copy_comps(P, mask, comps, [P](int c, const double *p) { return upload_comp(P, c, p, 8); });
+    if (rc != FDTD_OK) return rc;
     CK(cudaStreamSynchronize(P->stream));
     return FDTD_OK;
 }
@@ -1498,12 +1509,8 @@ int fdtd_set_fields_f32(fdtd_plan *P, int mask, const float *const comps[6])
 {
     if (!P || !comps) return fail(FDTD_E_INVALID, "NULL argument");
     CK(cudaSetDevice(P->device));
-    for (int c = 0; c < 6; c++) {
-        if (!(mask & (1 << c))) continue;
-        if (!comps[c]) return fail(FDTD_E_INVALID, "selected component pointer is NULL");
-        int rc = upload_comp(P, c, comps[c], 4);
-        if (rc != FDTD_OK) return rc;
-    }
+    const int rc = copy_comps(P, mask, comps, [P](int c, const float *p) { return upload_comp(P, c, p, 4); });
+    if (rc != FDTD_OK) return rc;
     // FP32 storage copies asynchronously
     if (P->storage != FDTD_STORE_F32) CK(cudaStreamSynchronize(P->stream));
     return FDTD_OK;
@@ -1513,12 +1520,8 @@ int fdtd_get_fields_f32(fdtd_plan *P, int mask, float *const comps[6])
 {
     if (!P || !comps) return fail(FDTD_E_INVALID, "NULL argument");
     CK(cudaSetDevice(P->device));
-    for (int c = 0; c < 6; c++) {
-        if (!(mask & (1 << c))) continue;
-        if (!comps[c]) return fail(FDTD_E_INVALID, "selected component pointer is NULL");
-        int rc = download_comp(P, c, comps[c], 4);
-        if (rc != FDTD_OK) return rc;
-    }
+    const int rc = copy_comps(P, mask, comps, [P](int c, float *p) { return download_comp(P, c, p, 4); });
+    if (rc != FDTD_OK) return rc;
     CK(cudaStreamSynchronize(P->stream));
     return device_error(P);
 }
@@ -1527,12 +1530,8 @@ int fdtd_get_fields(fdtd_plan *P, int mask, double *const comps[6])
 {
     if (!P || !comps) return fail(FDTD_E_INVALID, "NULL argument");
     CK(cudaSetDevice(P->device));
-    for (int c = 0; c < 6; c++) {
-        if (!(mask & (1 << c))) continue;
-        if (!comps[c]) return fail(FDTD_E_INVALID, "selected component pointer is NULL");
-        int rc = download_comp(P, c, comps[c], 8);
-        if (rc != FDTD_OK) return rc;
-    }
+    const int rc = copy_comps(P, mask, comps, [P](int c, double *p) { return download_comp(P, c, p, 8); });
+    if (rc != FDTD_OK) return rc;
     CK(cudaStreamSynchronize(P->stream));
     return device_error(P);
 }

@@ -68,3 +68,23 @@ def test_staging_is_made_by_the_first_copy_that_converts():
     assert b >= a - (2 << 20)
     assert 8 * n ** 3 - (2 << 20) <= b - c <= 8 * n ** 3 + (2 << 20)
     assert d >= c - (2 << 20)
+
+
+def test_error_returns_after_the_copies_queued_before_it():
+    """Page-locked arrays, so that the copies are the device's alone (16 M cells: ms)."""
+    shape = (256, 256, 256)
+    s = plan.Scene(name="copy", xres=256, yres=256, zres=256, dx=10e-9, dt=plan.plan_dt(10e-9, 10e-9, 10e-9, 0.5), nsteps=1)
+    s.mats = [plan.vacuum_material()]
+    s.mat = np.zeros(shape, dtype=np.int32)
+    st = torch.cuda.Stream()
+    with Solver(s) as g:
+        g.set_stream(st.cuda_stream)
+        for dt, ct in ((torch.float64, C.c_double), (torch.float32, C.c_float)):
+            host = torch.zeros(shape, dtype=dt).pin_memory().numpy()
+            p = abi.field_ptrs([host, None, None, None, None, None], ct)
+            f32 = "_f32" if dt == torch.float32 else ""
+            for fn in ("fdtd_set_fields" + f32, "fdtd_get_fields" + f32):
+                with pytest.raises(abi.FdtdError, match="NULL"):
+                    abi.check(getattr(g.lib, fn)(g.h, 3, p), fn)
+                assert st.query(), fn
+        g.set_stream(None)
