@@ -104,7 +104,9 @@ struct fdtd_plan {
     // and the flat kernels on the rest, or the flat kernels on the whole grid
     int fwidth = 1;                          // cells per thread of the flat kernels
     std::vector<FlatBlock> h_flat;           // host copy of their block list (batched launches)
-    FlatList flat, flat_in, flat_sp;         // all blocks; the plain interior's and the rest (fdtd_step_profile)
+    FlatList flat;                           // all blocks
+    FlatList flat_in, flat_sp;               // the plain interior's and the rest (profile_parts)
+    bool parts = false;
     BulkItem *d_bulk = nullptr;
     int nbulk = 0;
     bool bulk_on = false;
@@ -132,11 +134,11 @@ struct fdtd_plan {
     int *d_err = nullptr;                 // set by a bulk CTA whose bounded wait expired
     const int *batch_err = nullptr;       // the batch's error word, for an instance of a batch
     bool failed = false;                  // an expired wait was reported: the plan only accepts destroy
-    int region[6] = {0, 0, 0, 0, 0, 0};   // bulk box Xlo Xhi Ylo Yhi Zlo Zhi
+    int region[6] = {0, 0, 0, 0, 0, 0};   // bulk box (the plain interior without a bulk kernel) Xlo Xhi Ylo Yhi Zlo Zhi
     std::vector<BulkItem> h_bulk;
     int bulk_len = 0;                     // planes per bulk item
     int tsf_cells = 0;                    // face cells of the TSF correction tables
-    double bulk_bytes = 0, slab_bytes = 0; // algorithmic HBM bytes per launch
+    double bulk_bytes = 0, slab_bytes = 0; // algorithmic HBM bytes a step of the interior and the rest (profile_parts)
     // NFFF
     bool nfff = false;
     int nfff_npoints = 0, nfff_nfreq = 0, nfff_ns = 0;
@@ -762,6 +764,64 @@ std::vector<FlatBlock> flat_blocks(const HostPlan &hp, const DevPlan &d, const i
     return flat_emit(pieces);
 }
 
+cudaError_t flat_upload(fdtd_plan *P, const std::vector<FlatBlock> &v, FlatList *l)
+{
+    FlatBlock *dv = nullptr;
+    l->n = (unsigned)v.size();
+    if (v.empty()) return cudaSuccess;
+    const cudaError_t e = upload(P->mem, &dv, v.data(), v.size());
+    l->blocks = dv;
+    return e;
+}
+
+// What fdtd_step_profile alone needs, made by its first call (creating a plan:
+// 100^3 28.8 -> 22.7 ms, 256^3 345 -> 335): the block lists of the interior and of
+// the rest, and their algorithmic bytes per step -- 24 B field reads + 24 B writes
+// + 1 class byte per cell; 12 B (Q read + write, E^{n-1} read) + 16 B per pole
+// per dispersive field component; 4 psi arrays x (4 B read + 4 B write) per
+// CPML cell (the rest only); at FP32, the others by their element size.
+cudaError_t profile_parts(fdtd_plan *P)
+{
+    if (P->parts) return cudaSuccess;
+    const HostPlan &hp = P->hp;
+    std::vector<FlatBlock> part[2];   // the rest, the interior
+    for (const FlatBlock &b : P->h_flat) part[(b.flags & FB_INNER) != 0].push_back(b);
+    const bool inner = P->bulk_on || !part[1].empty();
+    const double esz = (double)P->esz;
+    std::vector<double> per(hp.classes.size());
+    for (size_t c = 0; c < per.size(); c++) {
+        const unsigned f = hp.classes[c].flags;
+        per[c] = 12.0 * esz + 1.0;
+        if (f & CF_ADE_BRANCH)
+            per[c] += (((f & CF_ADE_X) ? 1 : 0) + ((f & CF_ADE_Y) ? 1 : 0) + ((f & CF_ADE_Z) ? 1 : 0)) * (8.0 + esz + 16.0 * hp.maxpoles);
+    }
+    const int *r = P->region;
+    double all = 0, in = 0;
+#pragma omp parallel for reduction(+ : all, in) schedule(static)
+    for (int i = 0; i < hp.xr; i++)
+        for (int j = 0; j < hp.yr; j++) {
+            const uint8_t *row = &hp.cls[((size_t)i * hp.yr + j) * hp.zr];
+            const bool plain = inner && i >= r[0] && i < r[1] && j >= r[2] && j < r[3];
+            double a = 0, b = 0;
+            for (int k = 0; k < hp.zr; k++) a += per[row[k]];
+            for (int k = r[4]; plain && k < r[5]; k++) b += per[row[k]];
+            all += a;
+            in += b;
+        }
+    for (int f = 0; f < 6; f++) {
+        if (!hp.cp[f].enabled) continue;
+        const double face = f < 2 ? (double)hp.yr * hp.zr : f < 4 ? (double)hp.xr * hp.zr : (double)hp.xr * hp.yr;
+        all += face * hp.cp[f].depth * 4 * 2.0 * esz;
+    }
+    P->bulk_bytes = in;
+    P->slab_bytes = all - in;
+    cudaError_t e = flat_upload(P, part[0], &P->flat_sp);
+    if (e == cudaSuccess) e = flat_upload(P, part[1], &P->flat_in);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();   // (the copies are on another stream)
+    P->parts = e == cudaSuccess;
+    return e;
+}
+
 void side_free(fdtd_plan *P)
 {
     for (cudaStream_t s : {P->prep, P->post})
@@ -1249,53 +1309,11 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
             const int planes = hi[0] - lo[0], nch = std::max(1, (planes + 9) / 10), len = (planes + nch - 1) / nch;
             blk = bulk_items(lo, hi, len, 0);
             P->bulk_len = len;
-            for (int ax = 0; ax < 3; ax++) { P->region[2 * ax] = lo[ax]; P->region[2 * ax + 1] = hi[ax]; }
         }
+        for (int ax = 0; ax < 3; ax++) { P->region[2 * ax] = lo[ax]; P->region[2 * ax + 1] = hi[ax]; }
         if ((double)hp.n / P->fwidth / FLAT_NT > 1.0e9) return bail(cudaErrorInvalidValue, "grid too large for the flat kernels");
         P->h_flat = flat_blocks(hp, d, lo, hi, !P->bulk_on, P->fwidth);
-        std::vector<FlatBlock> part[2];   // the rest, the interior
-        for (const FlatBlock &b : P->h_flat) part[(b.flags & FB_INNER) != 0].push_back(b);
-        const bool inner = P->bulk_on || !part[1].empty();
-        {
-            auto list = [&](const std::vector<FlatBlock> &v, FlatList *l) {
-                FlatBlock *dv = nullptr;
-                l->n = (unsigned)v.size();
-                if (v.empty()) return cudaSuccess;
-                cudaError_t e = upload(P->mem, &dv, v.data(), v.size());
-                l->blocks = dv;
-                return e;
-            };
-            CA(list(P->h_flat, &P->flat), "flat blocks");
-            CA(list(part[0], &P->flat_sp), "flat blocks");
-            CA(list(part[1], &P->flat_in), "flat blocks");
-        }
-        {   // algorithmic bytes per step of the interior and of the rest: 24 B field reads + 24 B writes
-            // + 1 class byte per cell; 12 B (Q read + write, E^{n-1} read) + 16 B per pole per dispersive
-            // field component; 4 psi arrays x (4 B read + 4 B write) per CPML cell (the rest only)
-            auto cell_bytes = [&](int i0, int i1, int j0, int j1, int k0, int k1) {
-                double b = 0;
-                if (i0 >= i1 || j0 >= j1 || k0 >= k1) return b;
-#pragma omp parallel for reduction(+ : b) schedule(static)
-                for (int i = i0; i < i1; i++)
-                    for (int j = j0; j < j1; j++)
-                        for (int k = k0; k < k1; k++) {
-                            const DevClass &c = hp.classes[hp.cls[((size_t)i * Y + j) * Z + k]];
-                            b += 12.0 * esz + 1.0;
-                            if (c.flags & CF_ADE_BRANCH)
-                                b += (((c.flags & CF_ADE_X) ? 1 : 0) + ((c.flags & CF_ADE_Y) ? 1 : 0) + ((c.flags & CF_ADE_Z) ? 1 : 0)) *
-                                     (8.0 + esz + 16.0 * hp.maxpoles);
-                        }
-                return b;
-            };
-            double psi = 0;
-            for (int f = 0; f < 6; f++)
-                if (hp.cp[f].enabled) {
-                    const int dep = hp.cp[f].depth;
-                    psi += ((f < 2) ? (double)dep * Y * Z : (f < 4) ? (double)X * dep * Z : (double)X * Y * dep) * 4 * 2.0 * esz;
-                }
-            P->bulk_bytes = inner ? cell_bytes(lo[0], hi[0], lo[1], hi[1], lo[2], hi[2]) : 0;
-            P->slab_bytes = cell_bytes(0, X, 0, Y, 0, Z) - P->bulk_bytes + psi;
-        }
+        CA(flat_upload(P, P->h_flat, &P->flat), "flat blocks");
         CA(P->mem.alloc(&P->d_err, 1), "error word");
         if (P->bulk_on) {
             CA(upload(P->mem, &P->d_bulk, blk.data(), blk.size()), "work table");
@@ -1691,6 +1709,7 @@ int fdtd_step_profile(fdtd_plan *P, int nsteps, double out[8])
     if (!P || nsteps < 1 || !out) return fail(FDTD_E_INVALID, "bad argument");
     if (P->failed) return refuse_failed(P);
     CK(cudaSetDevice(P->device));
+    if (!P->tiles_on) CK(profile_parts(P));
     const int NE = 6;
     std::vector<cudaEvent_t> ev((size_t)NE * nsteps);
     for (auto &e : ev) CK(cudaEventCreate(&e));

@@ -1,36 +1,15 @@
-"""A launch that fails in the middle of a stepping call, from a fake of the failing
-runtime call in a child process (nothing is launched in its place): the plan
-stays at the last step queued whole, its field set, step count, device counter
-(probe rows), far-field sums and replay graphs agreeing, and steps on from there
-to the bits of a run without the failure.  The scene has no TSF box: the 1D grid
-alone runs ahead of the steps."""
-import os
-import subprocess
-import sys
+"""Through a fake of a runtime call, in a child process.
 
+A launch that fails in the middle of a stepping call (nothing is launched in its
+place): the plan stays at the last step queued whole, its field set, step count,
+device counter (probe rows), far-field sums and replay graphs agreeing, and steps
+on from there to the bits of a run without the failure.  The scene has no TSF
+box: the 1D grid alone runs ahead of the steps."""
 import pytest
 
-pytestmark = pytest.mark.gpu
-ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+from tests._fakecuda import run_child
 
-FAKE = r"""
-#define _GNU_SOURCE
-#include <dlfcn.h>
-static int left, pending;
-void fake_arm(int k) { left = k; }            /* the k-th launch of the flat E kernel from now fails */
-static void *real(const char *n) { return dlsym(dlopen("libcudart.so.12", RTLD_NOW | RTLD_NOLOAD), n); }
-int cudaLaunchKernelExC(const void *c, const void *f, void **a)
-{
-    if (left > 0 && --left == 0) return pending = 701;   /* cudaErrorLaunchOutOfResources */
-    return ((int (*)(const void *, const void *, void **))real("cudaLaunchKernelExC"))(c, f, a);
-}
-int cudaGetLastError(void)
-{
-    int e = pending;
-    pending = 0;
-    return e ? e : ((int (*)(void))real("cudaGetLastError"))();
-}
-"""
+pytestmark = pytest.mark.gpu
 
 CHILD = r"""
 import ctypes, os, sys
@@ -71,9 +50,28 @@ print("agree")
 
 
 def test_plan_after_a_failed_launch(tmp_path):
-    src, so = tmp_path / "fake.c", tmp_path / "fake.so"
-    src.write_text(FAKE)
-    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(so), str(src), "-ldl"], check=True)
-    env = dict(os.environ, LD_PRELOAD=str(so), PYTHONPATH=ROOT)
-    r = subprocess.run([sys.executable, "-c", CHILD], env=env, cwd=ROOT, capture_output=True, text=True, timeout=120)
-    assert r.returncode == 0 and "agree" in r.stdout, r.stdout + r.stderr
+    run_child(CHILD, tmp_path)
+
+
+PROFILE = r"""
+import ctypes, os
+from gsvit_copy_b200 import plan
+from gsvit_copy_b200.solver import Solver
+fake = ctypes.CDLL(os.environ["LD_PRELOAD"])
+s = plan.small_scene("full", shape=(40, 52, 72))
+with Solver(s) as g:
+    made = fake.fake_mallocs()
+    g.step(2)
+    assert fake.fake_mallocs() == made
+    first = g.step_profile(1)
+    assert fake.fake_mallocs() == made + 2      # the block lists of the interior and of the rest
+    again = g.step_profile(1)
+    assert fake.fake_mallocs() == made + 2
+    assert first["bulk_bytes"] == again["bulk_bytes"] > 0 and first["slab_bytes"] == again["slab_bytes"] > 0
+print("agree")
+"""
+
+
+def test_profile_makes_its_own_lists(tmp_path):
+    """What fdtd_step_profile alone needs is made by its first call, not with the plan."""
+    run_child(PROFILE, tmp_path)
