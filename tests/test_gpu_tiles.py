@@ -20,7 +20,7 @@ TOL = 1e-5
 
 @pytest.fixture(autouse=True)
 def _tiles_on(monkeypatch):
-    """These CPML depths (6-12) take the slab kernels by default; force the tiles."""
+    """FP32 grids take the flat kernels by default; force the tiles."""
     monkeypatch.setenv("GSVIT_B200_TILES", "1")
 
 
@@ -64,10 +64,9 @@ def test_tiles_tsf_driven_farfield(kind, shape, depth):
     assert rel_l2(g.nfff_spectrum(), ref) < TOL
 
 
-def test_tiles_use_three_layouts_and_match_slab_path(monkeypatch):
-    """The same run through the tiles and through the slab kernels (the path of
-    plans without tiles, selected by GSVIT_B200_NO_BULK) agree to FP32
-    rounding; the tiled step launches the bulk and the three CPML kinds."""
+def test_tiles_use_three_layouts_and_match_flat_path(monkeypatch):
+    """The same run through the tiles and through the flat kernels alone (selected
+    by GSVIT_B200_NO_BULK) agree to FP32 rounding; the tiled step launches the bulk and the three CPML kinds."""
     s = tiled_scene("full", (40, 52, 72), 8, 40)
     init = random_fields((s.xres, s.yres, s.zres), 4)
     g = Solver(s)
