@@ -2299,21 +2299,24 @@ int fdtd_batch_tune(fdtd_batch *B, int trial_steps, double *report, int report_l
     if (!B || trial_steps < 1) return fail(FDTD_E_INVALID, "bad argument");
     CK(cudaSetDevice(B->device));
     CK(cudaStreamSynchronize(B->stream));
-    // keep the state: every plan's stepping state into one device backup
+    // keep the state: every plan's stepping state and probe rows into one device backup
+    std::vector<SnapItem> kept;
     size_t total = 0;
-    for (auto *P : B->plans)
-        for (auto &it : P->snap) total += it.bytes;
+    for (auto *P : B->plans) {
+        kept.insert(kept.end(), P->snap.begin(), P->snap.end());
+        if (P->aux.nprobes) kept.push_back({P->aux.probe_out, (size_t)P->aux.nprobes * 6 * P->aux.nsteps_planned * sizeof(double)});
+    }
+    for (auto &it : kept) total += it.bytes;
     char *backup = nullptr;
     CK(cudaMalloc(&backup, std::max<size_t>(total, 16)));
     auto copy_state = [&](bool save) -> cudaError_t {
         char *q = backup;
-        for (auto *P : B->plans)
-            for (auto &it : P->snap) {
-                cudaError_t e = save ? cudaMemcpyAsync(q, it.ptr, it.bytes, cudaMemcpyDeviceToDevice, B->stream)
-                                     : cudaMemcpyAsync(it.ptr, q, it.bytes, cudaMemcpyDeviceToDevice, B->stream);
-                if (e != cudaSuccess) return e;
-                q += it.bytes;
-            }
+        for (auto &it : kept) {
+            cudaError_t e = save ? cudaMemcpyAsync(q, it.ptr, it.bytes, cudaMemcpyDeviceToDevice, B->stream)
+                                 : cudaMemcpyAsync(it.ptr, q, it.bytes, cudaMemcpyDeviceToDevice, B->stream);
+            if (e != cudaSuccess) return e;
+            q += it.bytes;
+        }
         return cudaSuccess;
     };
     const int cur0 = B->cur;

@@ -19,7 +19,7 @@ def _scenes(nsteps):
           plan.rough_surface_scene(res=40, yres=72, zres=48, nsteps=nsteps, cpml_depth=8, tsf_margin=6, seed=4,
                                    nfff_angles=(4, 7)),
           plan.small_scene("full", nsteps=nsteps),
-          plan.small_scene("lintab", shape=(26, 22, 30), nsteps=nsteps)]   # zres % 4 != 0: slab kernels only
+          plan.small_scene("lintab", shape=(26, 22, 30), nsteps=nsteps)]   # zres % 4 != 0: one cell a thread, no bulk kernel
     return sc
 
 
@@ -55,18 +55,19 @@ def test_batch_matches_one_by_one_bitwise():
     batch.close()
 
 
-def test_batch_tune_keeps_state_and_results():
+def test_batch_tune_keeps_state_and_results(monkeypatch):
+    monkeypatch.setenv("GSVIT_B200_BULK", "1")
     n = 30
-    scenes = _scenes(n)
+    scenes = _scenes(50)     # rows of the trial steps past the run's end too
     batch = Batch(scenes)
     _init(batch.views, scenes)
     batch.step(10)
     report = batch.tune(trial_steps=2)
     assert len(report) == 10 and all(r[2] > 0 for r in report)
     cfg = batch.config()
-    # the bulk work list holds only the instances without TMA tiles (here the
-    # one whose zres is not a multiple of 4)
-    assert cfg["items"] >= 0 and cfg["planes_per_item"] in (0, 8, 16, 32, 64)
+    # the bulk work list holds the instances whose zres is a multiple of 4
+    assert cfg["items"] > 0 and cfg["planes_per_item"] in (0, 8, 16, 32, 64)
+    assert (cfg["planes_per_item"], bool(cfg["persistent"])) == min(report, key=lambda r: r[2])[:2]
     batch.step(20)
     batch.sync()
     for q, sc in enumerate(scenes):
