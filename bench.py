@@ -524,7 +524,8 @@ def storage_measure(res, storage, K, W, device):
 
 def batched_measure(K, W, nscenes=48, tune_steps=2):
     """The batched instances (plan.batch_scenes) stepped as one batch from CUDA
-    graphs after the tuner picked the bulk work list; device-synchronised host
+    graphs, after the tuner where the bulk kernel has work (these instances run
+    the flat kernels: it reports no candidates); device-synchronised host
     clock around K steps."""
     import torch
     from gsvit_copy_b200 import plan
@@ -569,7 +570,7 @@ def extensions(a, device):
 def run_batched(a):
     """48 independent rough-surface instances (x, y in {64, 96, 128, 192}, z in
     {64, 96, 128}, Drude or Lorentz, 8-cell CPML) stepped as one batch per GPU
-    after the autotuner picked its work list, against the same instances
+    (the autotuner has no candidates for them), against the same instances
     stepped one by one with the plain solver (each from a CUDA graph).  With N
     ranks (torchrun, one GPU each) the instances are split whole across the
     ranks (plan.shard_instances: no exchange, weak in the instance count per

@@ -2297,6 +2297,10 @@ int fdtd_batch_sync(fdtd_batch *B)
 int fdtd_batch_tune(fdtd_batch *B, int trial_steps, double *report, int report_len, int *ncand)
 {
     if (!B || trial_steps < 1) return fail(FDTD_E_INVALID, "bad argument");
+    if (ncand) *ncand = 0;
+    // The candidates are bulk work lists.  Without a bulk kernel (instances of less
+    // than 25 M cells at FP32, TMA tiles) they would be one step timed ten times.
+    if (!B->nitems[0] && !B->nitems[1] && !B->nitems[2]) return FDTD_OK;
     CK(cudaSetDevice(B->device));
     CK(cudaStreamSynchronize(B->stream));
     // keep the state: every plan's stepping state and probe rows into one device backup

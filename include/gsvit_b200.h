@@ -369,10 +369,11 @@ int fdtd_batch_step_graph(fdtd_batch *batch, int nsteps, int chunk);
 int fdtd_batch_sync(fdtd_batch *batch);
 /* Autotuner: times trial_steps steps for each candidate work list of the
  * bulk kernel (planes per bulk item 8 / 16 / 32 / 64 / whole, persistent grid
- * or one CTA per item; it steps the instances without TMA tiles), keeps the
- * fastest and restores every instance's state.  report (if not NULL)
- * receives up to report_len/3 rows {planes (0 = whole), persistent, ms per
- * step}; *ncand the number of rows. */
+ * or one CTA per item), keeps the fastest and restores every instance's state
+ * and probe rows.  report (if not NULL) receives up to report_len/3 rows
+ * {planes (0 = whole), persistent, ms per step}; *ncand the number of rows: 0
+ * for a batch without work for the bulk kernel (FP32 instances of less than
+ * 25,165,824 cells), where there is nothing to pick. */
 int fdtd_batch_tune(fdtd_batch *batch, int trial_steps, double *report, int report_len, int *ncand);
 /* The bulk work list in use: planes per item (0 = whole), persistent launch,
  * grid size and number of items. */

@@ -79,6 +79,17 @@ def test_batch_tune_keeps_state_and_results(monkeypatch):
     batch.close()
 
 
+def test_batch_tune_without_bulk_kernel_times_nothing():
+    batch = Batch(_scenes(4))
+    cfg = batch.config()
+    assert cfg["items"] == 0
+    assert batch.tune(trial_steps=2) == [] and batch.config() == cfg
+    batch.step(2)
+    batch.sync()
+    assert batch[0].step_count == 2 and not batch[0].probes()[:, 2:].any()
+    batch.close()
+
+
 def test_batch_lorentz_instance_vs_oracle():
     n = 160
     scenes = _scenes(n)
