@@ -1,8 +1,8 @@
 """The far-field kernels at the sizes where they can go wrong, against the FP64
 oracle: one frequency, a full group of them and one more; points whose
 retarded time falls on an integer (diagonals of the grid, where the Courant
-ratio is rational), points in a surface cell itself, more points than a CTA
-takes.  Relative L2 1e-5, as the other far-field tests (FP32 fields)."""
+ratio is rational), points in a surface cell itself, points of a block's second
+half alone (129), one more than a block takes (257), a second block in part.  Relative L2 1e-5, as the other far-field tests (FP32 fields)."""
 import numpy as np
 import pytest
 
@@ -35,7 +35,8 @@ DIAGONAL = [(6 + 40 * q, 6 + 40 * q, 6 + 40 * q) for q in range(1, 9)]
 
 
 @pytest.mark.parametrize("nfreq", [1, 2, 3, 4, 5, 8, 9])
-@pytest.mark.parametrize("points", [DIAGONAL, _sphere(129, 90), _sphere(5, 3000)], ids=["diagonal", "near", "far"])
+@pytest.mark.parametrize("points", [DIAGONAL, _sphere(129, 90), _sphere(5, 3000), _sphere(257, 90), _sphere(400, 400)],
+                         ids=["diagonal", "near", "far", "two_blocks", "two_blocks_far"])
 def test_spectrum(points, nfreq):
     s = _scene(points, nfreq)
     g, o = Solver(s), CpuSolver(s)
