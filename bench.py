@@ -266,9 +266,15 @@ def ncu_traffic(res, kernel="bulk_kernel"):
     return None
 
 
+FLAT = "flat_h_kernel + flat_e_kernel "
+# what stepped the interior and the rest of the grid, by the field kernels of a
+# step: TMA tiles (bulk and three CPML layouts), bulk and flat H and E, flat H and E
 KERNEL_NAMES = {
-    "bulk": "tile_kernel, bulk layout (TMA-staged fused H+E step of the interior box)",
-    "cpml": "flat_h_kernel + flat_e_kernel (the cells around the interior: psi, kappa and ADE-in-CPML)",
+    4: ("tile_kernel, bulk layout (TMA-staged fused H+E step of the interior box)",
+        "tile_kernel, CPML layouts (TMA-staged fused H+E step with psi, kappa and ADE-in-CPML)"),
+    3: ("tile_kernel, bulk layout (TMA-staged fused H+E step of the interior box)",
+        FLAT + "(the cells around the interior: psi, kappa and ADE-in-CPML)"),
+    2: (FLAT + "(the plain interior)", FLAT + "(the cells around the interior: psi, kappa and ADE-in-CPML)"),
 }
 
 
@@ -276,14 +282,17 @@ def kernel_rooflines(prof, nprof, step_bytes, step_ms, peak, peak_kind, res):
     """Per-kernel figures of one step from fdtd_step_profile (CUDA events
     around each launch group): device ms, algorithmic bytes, achieved GB/s and
     the fraction of the HBM peak; the roofline block is the kernel with the
-    largest share of the step."""
+    largest share of the step.  (The scene has a TSF and an NFFF box: four of a
+    step's launches are not field kernels.)"""
     total = prof["total_ms"] / nprof
+    field_kernels = int(prof["launches_per_step"]) - 4
+    names = dict(zip(("bulk", "cpml"), KERNEL_NAMES.get(field_kernels, KERNEL_NAMES[4])))
     ks = {}
     for key, ms_key, b_key in (("bulk", "bulk_ms", "bulk_bytes"), ("cpml", "slab_ms", "slab_bytes")):
         ms = prof[ms_key] / nprof
         b = prof[b_key]
         gbs = b / (ms * 1e-3) / 1e9 if ms > 0 else None
-        ks[key] = {"kernel": KERNEL_NAMES[key], "ms_per_launch": ms, "algorithmic_bytes": b, "achieved_gbs": gbs,
+        ks[key] = {"kernel": names[key], "ms_per_launch": ms, "algorithmic_bytes": b, "achieved_gbs": gbs,
                    "frac": gbs / peak if gbs else None, "step_share": ms / total if total else None}
     ks["aux_tsf"] = {"kernel": "1D aux grid + TSF face tables", "ms_per_step": prof["aux_ms"] / nprof,
                      "step_share": prof["aux_ms"] / nprof / total if total else None}
@@ -293,7 +302,7 @@ def kernel_rooflines(prof, nprof, step_bytes, step_ms, peak, peak_kind, res):
     t = ks[top]
     roofline = {"kernel": t["kernel"], "bound": "hbm", "achieved": t["achieved_gbs"], "peak": peak, "unit": "GB/s",
                 "frac": t["frac"], "peak_source": peak_kind,
-                "traffic": ncu_traffic(res) if top == "bulk" else None,
+                "traffic": ncu_traffic(res) if top == "bulk" and field_kernels > 2 else None,
                 "algorithmic_bytes": t["algorithmic_bytes"], "ms_per_launch": t["ms_per_launch"],
                 "step_share": t["step_share"]}
     step_gbs = step_bytes / (step_ms * 1e-3) / 1e9
@@ -435,8 +444,8 @@ def run_b200(a):
     t0 = time.perf_counter()
     spec = g.nfff_spectrum()
     ff_ms = (time.perf_counter() - t0) * 1e3
-    # the step kernels of K steps, then the probe capture that closes fdtd_step
-    gpu_launches = int(prof["launches_per_step"]) * K + (1 if scene.probes is not None and len(scene.probes) else 0)
+    # the step kernels of K steps, and the one that closes each replayed chunk and the steps past the last
+    gpu_launches = int(prof["launches_per_step"]) * K + -(-K // GRAPH_CHUNK)
 
     # end to end through the public API with pinned host buffers
     shape = g.shape
