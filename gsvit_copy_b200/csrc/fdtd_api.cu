@@ -1,10 +1,12 @@
 // fdtd_api.cu -- the C ABI of include/gsvit_b200.h.
 //
-// Owns the device state of one plan and sequences the kernels of a step on a
-// single CUDA stream.  The reference's GPU driver (gpu.c) keeps a worker
-// thread per GPU, pushes one token per stage and spins on the host after
-// every launch (gpu.c:787-801, gpu_kernels.cu:6063-6068); here a step is
-// three stream-ordered launches with no host synchronisation, and
+// Owns the device state of one plan and sequences the kernels of its steps: the
+// field updates on the plan's stream, the next step's 1D grid and TSF tables and
+// the last step's NFFF work on two side streams joined by events.  The
+// reference's GPU driver (gpu.c) keeps a worker thread per GPU, pushes one token
+// per stage and spins on the host after every launch (gpu.c:787-801,
+// gpu_kernels.cu:6063-6068); here a step is about six launches (1D grid, TSF
+// faces, H, E, NFFF sampling and fold) with no host synchronisation, and
 // fdtd_step_graph replays them from a CUDA graph.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -201,10 +203,10 @@ DevPlan plan_for(const fdtd_plan *P, int in)
     return d;
 }
 
-// one launch of the tile kernel of `kind` (TILE_*) for this step's parity
 // the variant of the flat E kernel: what the dispersive state can hold
 int flat_poles(const fdtd_plan *P) { return P->one_pole ? 1 : P->hp.maxpoles; }
 
+// one launch of the tile kernel of `kind` (TILE_*) for this step's parity
 int launch_tile_kind(fdtd_plan *P, const DevPlan &d, int in, int kind, cudaStream_t st)
 {
     const cudaError_t e = launch_tiles(kind, d, P->tmaps[kind][in], P->d_tiles[kind], P->ntiles[kind], P->d_err,
@@ -422,7 +424,7 @@ std::vector<BulkItem> bulk_items(const int lo[3], const int hi[3], int len, int 
 }
 
 
-int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool pole_arrays);
+int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out);
 
 // The largest run [a, b) of indices along one axis whose cells take the plain
 // update (hp.ike/ikh of 1, outside the CPML psi ranges of boundary.c:347-519
@@ -500,14 +502,12 @@ extern "C" {
 
 const char *fdtd_last_error(void) { return g_err.c_str(); }
 
-int fdtd_plan_create(const fdtd_desc *desc, int device, fdtd_plan **out) { return plan_create_impl(desc, device, out, false); }
+int fdtd_plan_create(const fdtd_desc *desc, int device, fdtd_plan **out) { return plan_create_impl(desc, device, out); }
 
 }  // extern "C"
 
 namespace {
 
-// pole_arrays: allocate the critical-point state even for a Drude-only plan,
-// so that a batched launch may run it with the two-pole kernel variant
 // Work lists of the TMA tile kernels for a single plan.  The interior box
 // (every index plain on every axis, the bulk tile's halo row, group and plane
 // plain for H) goes to the bulk layout, its last tiles partial; the rest of
@@ -830,7 +830,7 @@ void side_free(fdtd_plan *P)
         if (e) cudaEventDestroy(e);
 }
 
-int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool pole_arrays)
+int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out)
 {
     if (!out) return fail(FDTD_E_INVALID, "out is NULL");
     *out = nullptr;
@@ -844,7 +844,6 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
         return fail(rc, err);
     }
     HostPlan &hp = P->hp;
-    if (pole_arrays && hp.has_ade) hp.maxpoles = 2;
     P->one_pole = hp.one_pole;
     P->storage = desc->storage;
     P->esz = desc->storage == FDTD_STORE_F32 ? 4 : desc->storage == FDTD_STORE_F64 ? 8 : 2;
@@ -1198,9 +1197,10 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out, bool po
             CA(upload(P->mem, &dtw, tw.data(), tw.size()), "far-field twiddles");
             int nsm = 148;
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-            // groups of surface cells: blocks for whole waves at 2, 3 or 6 blocks an SM (1, 3 and 4
-            // frequencies a launch; 192^3, 4186 points: 10.3 ms at 2.1 blocks an SM, 7.0 at 6, 6.9 at 12),
-            // in partial sums of 256 MB at most where that leaves blocks for four an SM
+            // groups of surface cells: six blocks an SM, whole waves for 1, 3 and 4 frequencies a launch
+            // (6, 3 and 2 blocks an SM at 80, 168 and 250 registers; 2 frequencies, at 4 an SM, run one wave
+            // and a half; 192^3, 4186 points, 3 frequencies: 10.3 ms at 2.1 blocks an SM, 7.0 at 6, 6.9 at
+            // 12), in partial sums of 256 MB at most where that leaves blocks for four an SM
             const int ptiles = (f.npoints + FF_TILE - 1) / FF_TILE;
             const size_t row = (size_t)f.npoints * f.nfreq * 3 * sizeof(double2);
             const int least = (4 * nsm + ptiles - 1) / ptiles;
@@ -2106,7 +2106,7 @@ int fdtd_batch_create(const fdtd_desc *descs, int nplans, int device, fdtd_batch
     if (cudaStreamCreateWithFlags(&B->stream, cudaStreamNonBlocking) != cudaSuccess) { delete B; return fail(FDTD_E_CUDA, "stream"); }
     for (int q = 0; q < nplans; q++) {
         fdtd_plan *P = nullptr;
-        const int rc = plan_create_impl(&descs[q], device, &P, false);
+        const int rc = plan_create_impl(&descs[q], device, &P);
         if (rc != FDTD_OK) {
             const std::string m = fdtd_last_error();
             batch_free(B);

@@ -106,16 +106,6 @@ __device__ __forceinline__ double ld_any(const float *p, int64_t i, int storage)
     return p[i];
 }
 
-// three components of the arithmetic type R (float3 / double3)
-template <class R>
-struct V3t;
-template <>
-struct V3t<float> { using type = float3; };
-template <>
-struct V3t<double> { using type = double3; };
-template <class R>
-using V3 = typename V3t<R>::type;
-
 // ---- coefficient tables of the arithmetic type R.  R = float reads the
 // FP32 tables of DevPlan; R = double (FDTD_STORE_F64 plans) reads the FP64
 // tables the same pointers then hold.
@@ -173,9 +163,9 @@ struct Tab<double> {
     __device__ static const DevAde64 &ade(const DevPlan &P, int a) { return reinterpret_cast<const DevAde64 *>(P.ade)[a]; }
 };
 
-// E (unscaled), H (times hs), psi_H (times ps) and psi_E (times pse) element
-// access.  Stores take the step number `stp` (sr_step) and the array index of
-// sr_seed, which only stochastic rounding uses.
+// Stores of an element take the step number `stp` (sr_step) and the array index
+// of sr_seed, which only stochastic rounding uses.  E is stored as it is, H
+// times hs, psi_H times ps and psi_E times pse (the caller scales).
 template <class T>
 __device__ __forceinline__ uint32_t sr_step(const DevPlan &P)
 {
@@ -190,63 +180,6 @@ __device__ __forceinline__ void st_any(float *p, int64_t i, typename Stor<T>::re
 }
 template <class T>
 using real_t = typename Stor<T>::real;
-template <class T>
-__device__ __forceinline__ real_t<T> ldE(const float *p, int64_t i) { return Stor<T>::ld(p, i); }
-template <class T>
-__device__ __forceinline__ real_t<T> ldgE(const float *p, int64_t i) { return Stor<T>::ldg(p, i); }
-template <class T>
-__device__ __forceinline__ void stE(float *p, int64_t i, real_t<T> v, uint32_t stp, uint32_t array)
-{
-    st_any<T>(p, i, v, stp, array);
-}
-template <class T>
-__device__ __forceinline__ real_t<T> ldH(const DevPlan &P, const float *p, int64_t i)
-{
-    if constexpr (Stor<T>::scaled) return Stor<T>::ld(p, i) * P.ihs;
-    else return Stor<T>::ld(p, i);
-}
-template <class T>
-__device__ __forceinline__ real_t<T> ldgH(const DevPlan &P, const float *p, int64_t i)
-{
-    if constexpr (Stor<T>::scaled) return Stor<T>::ldg(p, i) * P.ihs;
-    else return Stor<T>::ldg(p, i);
-}
-template <class T>
-__device__ __forceinline__ void stH(const DevPlan &P, float *p, int64_t i, real_t<T> v, uint32_t stp, uint32_t array)
-{
-    if constexpr (Stor<T>::scaled) st_any<T>(p, i, v * P.hs, stp, array);
-    else st_any<T>(p, i, v, stp, array);
-}
-template <class T>
-__device__ __forceinline__ real_t<T> ldPsi(const DevPlan &P, const float *p, int64_t i)
-{
-    if constexpr (Stor<T>::scaled) return Stor<T>::ld(p, i) * P.ips;
-    else return Stor<T>::ld(p, i);
-}
-template <class T>
-__device__ __forceinline__ real_t<T> ldgPsi(const DevPlan &P, const float *p, int64_t i)
-{
-    if constexpr (Stor<T>::scaled) return Stor<T>::ldg(p, i) * P.ips;
-    else return Stor<T>::ldg(p, i);
-}
-template <class T>
-__device__ __forceinline__ void stPsi(const DevPlan &P, float *p, int64_t i, real_t<T> v, uint32_t stp, uint32_t array)
-{
-    if constexpr (Stor<T>::scaled) st_any<T>(p, i, v * P.ps, stp, array);
-    else st_any<T>(p, i, v, stp, array);
-}
-template <class T>
-__device__ __forceinline__ real_t<T> ldPsiE(const DevPlan &P, const float *p, int64_t i)
-{
-    if constexpr (Stor<T>::scaled) return Stor<T>::ld(p, i) * P.ipse;
-    else return Stor<T>::ld(p, i);
-}
-template <class T>
-__device__ __forceinline__ void stPsiE(const DevPlan &P, float *p, int64_t i, real_t<T> v, uint32_t stp, uint32_t array)
-{
-    if constexpr (Stor<T>::scaled) st_any<T>(p, i, v * P.pse, stp, array);
-    else st_any<T>(p, i, v, stp, array);
-}
 
 // a hint that moves the line holding p into L2; no register, no wait
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -339,10 +272,6 @@ template <class T>
 __device__ __forceinline__ void stg4a(float *base, int64_t c, const float (&v)[4], float scale, uint32_t stp, uint32_t array)
 {
     stg4<T>(base, c, make_float4(v[0], v[1], v[2], v[3]), scale, stp, array);
-}
-__device__ __forceinline__ void lds4a_f(float (&d)[4], const float4 v)
-{
-    d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
 }
 // FP32 state arrays (ADE)
 __device__ __forceinline__ void ldq4a(float (&d)[4], const float *p)
