@@ -1,7 +1,7 @@
 // fdtd_adjoint.cu -- discrete adjoint of one source-free FDTD step.
 //
-// No counterpart in the reference.  The forward step of the general path
-// (slab kernels; the bulk kernel computes the same expressions) is linear in
+// No counterpart in the reference.  The forward step (flat kernels; the bulk
+// kernel computes the same expressions) is linear in
 // (E, H, psi_E, psi_H): the H half step (ystep_h yee.c:146-265, CPML H
 // boundary.c:347-519, zero planes boundary.c:418-492) and the E half step
 // (ystep_e yee.c:530-1247 with the dispersive branch in the difference form of

@@ -926,7 +926,12 @@ constexpr int H_AHEAD = 1536, E_AHEAD = 1024;
 
 // Resident blocks asked for.  H: 24 warps an SM at 80 registers (20 at 88:
 // 256^3 rough surface 405 -> 393 us a step).  E: 16 warps at 128; 20 warps spill
-// the dispersive variant (403 us).  Single cells: 40 and 28 warps.
+// the dispersive variant (403 us).  Single cells: 40 and 28 warps.  What still
+// spills (bytes a thread, stores / loads): E of groups with two poles 48 / 112, H
+// of groups 32 / 56, BF16 H 156 / 212; the batch forms, which read the plan
+// through a pointer, 140 / 428 with two poles; FP64 single cells, whose bounds are
+// FP32's, up to 1664 / 1696 with two poles (96 x 96 x 97, metal in half of it: 99
+// us a step, 170 with the kernels of one cell a thread before).
 template <int V>
 constexpr int H_BLOCKS = V == 1 ? 10 : 6;
 template <int V>

@@ -426,7 +426,9 @@ int fdtd_objective_value(fdtd_plan *plan, const fdtd_objective *obj, double *J);
  * region are transposed with their polarisation state.  On return the plan holds the
  * forward state after nsteps.  Device memory: (nsteps/checkpoint + 1) copies
  * of the stepping state (fdtd_snapshot_size) plus checkpoint x 12 bytes per
- * cell of the design box. */
+ * cell of the design box and the adjoint state (72 bytes a cell and more).  Up
+ * to 2 GB in all the plan keeps it for its next adjoint call and gives it back
+ * when it is destroyed; above that it is given back when the call returns. */
 int fdtd_adjoint_gradient(fdtd_plan *plan, const fdtd_objective *obj, int nsteps, int checkpoint,
                           double *J, double *grad);
 
