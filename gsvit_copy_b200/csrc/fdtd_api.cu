@@ -75,6 +75,10 @@ struct DevBuf {        // a list of device allocations freed with the plan
     }
 };
 
+// Waits for set-up work (DevBuf, upload: the default stream).  Not for the device:
+// that is refused, and spoils the capture, while another thread captures a graph.
+cudaError_t sync_setup() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 struct TsfTab {        // the TSF corrections of one step
     float2 *h[6], *e[6];
 };
@@ -817,7 +821,7 @@ cudaError_t profile_parts(fdtd_plan *P)
     P->slab_bytes = all - in;
     cudaError_t e = flat_upload(P, part[0], &P->flat_sp);
     if (e == cudaSuccess) e = flat_upload(P, part[1], &P->flat_in);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();   // (the copies are on another stream)
+    if (e == cudaSuccess) e = sync_setup();
     P->parts = e == cudaSuccess;
     return e;
 }
@@ -1370,7 +1374,7 @@ int plan_create_impl(const fdtd_desc *desc, int device, fdtd_plan **out)
         }
     }
     P->step_bytes = bytes;
-    CA(cudaDeviceSynchronize(), "plan set-up");
+    CA(sync_setup(), "plan set-up");
 #undef CA
     *out = P;
     return FDTD_OK;
@@ -2195,7 +2199,7 @@ int fdtd_batch_create(const fdtd_desc *descs, int nplans, int device, fdtd_batch
         }
     }
     BA(batch_set_items(B, 0, true), "batch work list");
-    BA(cudaDeviceSynchronize(), "batch set-up");
+    BA(sync_setup(), "batch set-up");
 #undef BA
     *out = B;
     return FDTD_OK;
