@@ -15,10 +15,11 @@
 //      update read (the curl and the psi recursions);
 //   B: per cell of the other field, the sum of the difference adjoints of the
 //      cells whose differences contain it.
-// Memory bounds them (A and B of both half steps move 192 bytes a cell): a thread
-// takes V consecutive k cells (4, or 1 on ragged rows) of a row, its block a
-// piece of a plane.  Plans with dispersive cells take A of the E half step a
-// cell a thread.  128 x 128 x 96, 12-cell CPML: 119 -> 59 us a transposed step.
+// They wait for memory (A and B of both half steps move 192 bytes a cell; A, with
+// 17 warps an SM, for its latency, B at half the DRAM peak): a thread takes V
+// consecutive k cells (4, or 1 on ragged rows) of a row, its block a piece of a
+// plane.  Plans with dispersive cells take A of the E half step a cell a thread.
+// 128 x 128 x 96, 12-cell CPML: 119 -> 59 us a transposed step.
 // Gates, coefficients and operation order follow flat_e_group / flat_h_group.
 #include <cuda_runtime.h>
 

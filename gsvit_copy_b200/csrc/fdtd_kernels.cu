@@ -382,9 +382,9 @@ __global__ void __launch_bounds__(128, 3) nfff_fold_batch(const DevNfff *N)
 //   w q cos(theta) (q + i kappa) * (-z Ehat / 4 pi)  +  w q * (sgn z Dhat / 4 pi),
 // kappa = sin(omega dt) / (c dt): the factors of a cell alone are formed when it
 // is staged, and the reference's square root and division run only for pairs
-// whose retarded index they could decide.  What bounds it is reading the staged
-// cells (each read serves the thread's FF_PTS points) and the table, then FP64
-// arithmetic (192^3, 4186 points, 3 frequencies: 13.9 ms with the factors formed
+// whose retarded index they could decide.  What bounds it is FP64 arithmetic (its
+// pipe 67 % busy, at 11 warps an SM that wait for its latency); each read of a
+// staged cell serves the thread's FF_PTS points (192^3, 4186 points, 3 frequencies: 13.9 ms with the factors formed
 // pair by pair, 11.7 with three staged terms and a point a thread, 7.0 now).
 constexpr int FF_PTS = FF_TILE / 128;
 
