@@ -60,7 +60,7 @@ def test_f16_e_follows_from_unrounded_h(shape, depth):
 
     Bound of a cell: half a unit of E in FP16 (2^-11 |E|), plus 1e-4 for the four
     H of a curl, each within a unit of FP32 (109 ohm times 4 2^-23 is 5.2e-5).  H
-    rounded to FP16 loses its update of 4e-5 A/m: 4e-3 V/m of E."""
+    rounded to FP16 loses its update, up to 2e-4 A/m here: 1e-2 V/m of E and more."""
     rng = np.random.default_rng(8)
     e0 = [(rng.integers(-1024, 1025, size=shape) * 2.0 ** -14).astype(np.float32) for _ in range(3)]   # FP16 numbers
     h0 = [np.ones(shape, dtype=np.float32)] * 3
